@@ -136,7 +136,7 @@ int32_t gblu_factor_set_solve(gblu_ctx* ctx, gblu_factor* f, int32_t mode);
 /* How a mixed-precision factor (GBLU_FP32 / BF16 / FP16) pivots its
  * low-precision LU, from the next getrf on (gblu_factor_set_pivoting).
  * GBLU_PIVOT_PARTIAL (default): partial pivoting, the reference's order
- *   (blocked_lufact.jl), per 32-column leaf.
+ *   (blocked_lufact.jl), leaf by leaf.
  * GBLU_PIVOT_TOURNAMENT: tournament pivoting (CALU's tall-skinny panel) for
  *   leaves taller than 512 rows.
  * GBLU_PIVOT_RBT: no pivoting, after a depth-2 random butterfly transform of

@@ -44,6 +44,16 @@ struct PanelSlots {
   T* diag_rowvals;   // [2][W]       current diagonal row
 };
 
+// A leaf's interchanges composed into row moves "row .x receives old row .y"
+// (matrix rows, 0-based), written by the panel kernel for the columns outside
+// the leaf: at most two per column of the leaf.
+constexpr int kLeafMaxW = 128;
+struct LeafMoves {
+  int32_t count;
+  int32_t pad[3];
+  int2 mv[2 * kLeafMaxW];
+};
+
 // ---------------------------------------------------------------------------
 // Host-side helpers
 
@@ -70,11 +80,12 @@ struct GetrfPlan {
   int32_t* perm = nullptr;   // device, length m: (P A)[i] = A[perm[i]]
   DevScratch* scratch = nullptr;
   PanelSlots<T> slots{};
-  int panel_width = 32;      // leaf width of the recursion
+  LeafMoves* moves = nullptr;  // the current leaf's interchanges (sub-panel kernel)
+  int panel_width = 32;      // leaf width of the recursion where the sub-panel kernel does not apply
   int panel_ctas = 0;        // CTAs of the cooperative panel kernel (0: auto)
   int trsm_base = 128;       // base size of the recursive TRSM
   bool use_cluster_panel = true;  // DSMEM cluster panel when the panel fits
-  bool use_reg_panel = true;      // register-resident cluster panel when the panel fits
+  bool use_sub_panel = true;      // sub-panel cluster kernel when the panel fits
   // FP32 working matrix only: trailing updates on tcgen05 with 16-bit operands
   int tc_mode = 0;           // 0 SIMT FP32, 1 BF16 operands, 2 FP16 operands (scaled)
   void* tc_work = nullptr;   // conversion buffers for the operands
@@ -107,6 +118,18 @@ cudaError_t tslu_panel_launch(float* A, int64_t lda, int64_t m, int64_t c0, int 
 // No-pivot leaf (GetrfPlan::nopivot); work: the tslu work area (its ticket).
 cudaError_t genp_panel_launch(float* A, int64_t lda, int64_t m, int64_t c0, int w, int64_t* ipiv,
                               int64_t* info, void* work, cudaStream_t s);
+
+// Sub-panel cluster kernel (panel.cu).  panel_sub_width: the leaf width it takes
+// for a leaf of M rows, 0 when it does not take it (or no cluster of 16 CTAs
+// can be launched).  The launch factors columns c0 .. c0 + w - 1 of rows
+// c0 .. m - 1 and leaves the leaf's interchanges in *moves.
+template <typename T>
+bool panel_sub_ready();
+template <typename T>
+int panel_sub_width(int64_t M);
+template <typename T>
+cudaError_t panel_sub_launch(T* A, int64_t lda, int64_t m, int64_t c0, int w, int64_t* ipiv, int64_t* info,
+                             LeafMoves* moves, DevScratch* scr, cudaStream_t s);
 
 // FP32 SIMT update C -= A * B in the reference's per-element order (getrf.cu).
 cudaError_t simt_gemm_sub_f32(int64_t M, int64_t N, int64_t K, const float* A, int64_t lda,

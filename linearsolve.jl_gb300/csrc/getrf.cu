@@ -339,392 +339,6 @@ panel_cluster_kernel(T* __restrict__ A, int64_t lda, int64_t m, int64_t c0, int 
   cluster.sync();  // no CTA leaves while another may still read its shared memory
 }
 
-template <typename T>
-struct Vec16;  // 16-byte vector of T
-template <>
-struct Vec16<float> {
-  using V = float4;
-  static constexpr int N = 4;
-  static __device__ __forceinline__ float get(const V& v, int e) { return e == 0 ? v.x : e == 1 ? v.y : e == 2 ? v.z : v.w; }
-  static __device__ __forceinline__ V make(const float* x) { return make_float4(x[0], x[1], x[2], x[3]); }
-};
-template <>
-struct Vec16<double> {
-  using V = double2;
-  static constexpr int N = 2;
-  static __device__ __forceinline__ double get(const V& v, int e) { return e == 0 ? v.x : v.y; }
-  static __device__ __forceinline__ V make(const double* x) { return make_double2(x[0], x[1]); }
-};
-
-template <typename T, int W>
-__device__ __forceinline__ void row_store(T* dst, const T (&src)[W]) {
-  using VT = Vec16<T>;
-#pragma unroll
-  for (int q = 0; q < W / VT::N; ++q) reinterpret_cast<typename VT::V*>(dst)[q] = VT::make(&src[q * VT::N]);
-}
-
-template <typename T, int W>
-__device__ __forceinline__ void row_load(T (&dst)[W], const T* src) {
-  using VT = Vec16<T>;
-#pragma unroll
-  for (int q = 0; q < W / VT::N; ++q) {
-    const typename VT::V v = reinterpret_cast<const typename VT::V*>(src)[q];
-#pragma unroll
-    for (int e = 0; e < VT::N; ++e) dst[q * VT::N + e] = VT::get(v, e);
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Register panel kernel: the same getf2 on rows [c0, m) x columns [c0, c0+w)
-// with every panel row held in registers by one thread for the whole leaf
-// (row base + tid + NT * r of CTA `cta`, r < RPT, the CTA holding R rows).
-// The registers rotate by one slot per column, identically in every thread,
-// so the current column is always slot 0 and the column loop is a plain loop
-// with one small body; rows are exchanged in slot order (16-byte shared
-// memory accesses, no index arithmetic).
-//
-// The CTAs exchange pivot candidates by pushing them: no cluster barrier per
-// column.  After the interchange and scaling of column k, each thread
-// updates only slot 1 (column k+1); each warp reduces its column-k+1
-// candidate and leaves it, with the candidate row and the diagonal row in
-// their partly updated form (slot 0 = the multiplier l, slot 1 updated,
-// slots 2.. not yet), in shared memory; the pushing warp (the last warp)
-// waits for them on a named barrier, reduces them to the CTA's candidate and
-// writes candidate, row and (in the diagonal row's CTA) the diagonal row into
-// every CTA's receive slots with st.async, each store counted by the
-// receiver's mbarrier of that column.  The other warps run the rest of the
-// update (slots 2..) meanwhile.  Warp 0 of every CTA waits on its own
-// mbarrier (a bounded wait), picks the winner among the G received
-// candidates, and finishes the update of the received pivot row and
-// diagonal row itself with the same fma(-l, u, a) on the same operands the
-// owners use, so they are bit-identical to the owners' registers; warp 1
-// computes 1 / |candidate| of every received candidate from its key (the bit
-// pattern of |a|) and hands the winner's to warp 0 through a named barrier.
-// One CTA barrier hands the pivot row to every thread.
-//
-// Receive slots are double-buffered by column parity.  A CTA pushes column
-// k+1 only after it received every CTA's column k, and each CTA pushes
-// column k only after it finished reading its column k-1 slots, so a push
-// never overwrites slots still being read.  Warps that hold no rows skip the
-// arithmetic (a predicated-off FP64 instruction still occupies the FP64
-// pipe).  The per-element arithmetic is panel_kernel's.
-constexpr int kRegPanelThreads = 512;
-
-// A CTA's pivot candidate as one 16-byte word: key, row (-1 = none), warp.
-template <typename K>
-__device__ __forceinline__ int4 cand_pack(K key, int row, int warp) {
-  if constexpr (sizeof(K) == 4) return make_int4((int)key, row, warp, 0);
-  else return make_int4((int)(unsigned)key, (int)(unsigned)(key >> 32), row, warp);
-}
-template <typename K>
-__device__ __forceinline__ void cand_unpack(const int4& c, K& key, int& row, int& warp) {
-  if constexpr (sizeof(K) == 4) { key = (K)(unsigned)c.x; row = c.y; warp = c.z; }
-  else { key = ((K)(unsigned)c.y << 32) | (K)(unsigned)c.x; row = c.z; warp = c.w; }
-}
-
-// The value whose bit pattern is the key (|a| for a key of a)
-template <typename T>
-__device__ __forceinline__ T key_magnitude(typename PivKey<T>::K key) {
-  if constexpr (sizeof(T) == 4) return __uint_as_float(key);
-  else return __longlong_as_double((long long)key);
-}
-
-// x with the sign of s (bit operations only)
-template <typename T>
-__device__ __forceinline__ T with_sign_of(T x, T s) {
-  if constexpr (sizeof(T) == 4)
-    return __uint_as_float(__float_as_uint(x) ^ (__float_as_uint(s) & 0x80000000u));
-  else
-    return __longlong_as_double(__double_as_longlong(x) ^
-                                (__double_as_longlong(s) & (long long)0x8000000000000000ull));
-}
-
-template <typename T, int RPT>
-__global__ void __launch_bounds__(kRegPanelThreads, 1)
-panel_reg_kernel(T* __restrict__ A, int64_t lda, int64_t m, int64_t c0, int w,
-                 int64_t* __restrict__ ipiv, int64_t* __restrict__ info_out, int R,
-                 DevScratch* __restrict__ scr) {
-  namespace cg = cooperative_groups;
-  using K = typename PivKey<T>::K;
-  using VT = Vec16<T>;
-  constexpr unsigned kAll = 0xffffffffu;
-  cg::cluster_group cluster = cg::this_cluster();
-  constexpr int NT = kRegPanelThreads, NW = NT / 32, W = kPanelMaxW;
-  constexpr int RB = W * (int)sizeof(T) / 16;  // 16-byte chunks per row
-  constexpr int kPusher = NW - 1;              // the warp that pushes the CTA's candidate
-  // [b]: column k uses buffer k & 1
-  __shared__ __align__(16) T s_crowv[2][NW][W];  // each warp's candidate row (published form)
-  __shared__ __align__(16) T s_diagv[2][W];      // the diagonal row (owner CTA, published form)
-  __shared__ __align__(16) T s_piv[2][W];        // the pivot row of column k, slot order of step k
-  __shared__ __align__(16) T s_old[W];           // the old diagonal row, for the pivot row's owner
-  __shared__ __align__(16) T r_row[2][16][W];    // received: CTA c's candidate row
-  __shared__ __align__(16) T r_diag[2][W];       // received: the diagonal row
-  __shared__ __align__(16) int4 r_cand[2][16];   // received: CTA c's candidate (cand_pack)
-  __shared__ __align__(8) unsigned long long r_bar[2];  // counts the received bytes of a column
-  __shared__ K s_cval[2][NW];
-  __shared__ int s_crow[2][NW];
-  __shared__ T s_rinv[16];                       // 1 / |candidate| of CTA c's candidate
-  __shared__ int s_p;
-  __shared__ T s_inv;
-
-  const int G = (int)cluster.num_blocks();
-  const int cta = (int)cluster.block_rank();
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t base = c0 + (int64_t)cta * R;
-  const int nloc = (int)max((int64_t)0, min((int64_t)R, m - base));
-  const bool warp_rows = warp * 32 < nloc;  // this warp holds at least one row
-  // bytes received per column: G candidates and rows, one diagonal row
-  const uint32_t rx_bytes = (uint32_t)(G * 16 * (1 + RB) + 16 * RB);
-  int* const err = &scr->error;
-  bool bad = false;  // a wait gave up: stop waiting, finish without hanging
-
-  T pr[RPT][W];  // slot j: column (k + j) mod 32 at step k
-#pragma unroll
-  for (int r = 0; r < RPT; ++r) {
-    const int i = tid + NT * r;
-#pragma unroll
-    for (int j = 0; j < W; ++j) pr[r][j] = (i < nloc && j < w) ? A[(base + i) + (c0 + j) * lda] : T(0);
-  }
-  if (tid == 0) {
-    pan_bar_init(pan_saddr(&r_bar[0]));
-    pan_bar_init(pan_saddr(&r_bar[1]));
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    pan_bar_arm(pan_saddr(&r_bar[0]), rx_bytes);  // column 0
-    pan_bar_arm(pan_saddr(&r_bar[1]), rx_bytes);  // column 1
-  }
-  cluster.sync();  // every CTA's mbarriers exist before the first push
-  int64_t info_local = 0;
-
-  // Candidates of the column in slot S among rows >= dn into buffer pb: each
-  // warp's first row of max |a| (NaN ignored) with its row, and the diagonal
-  // row dn; the pushing warp reduces them to the CTA's candidate and writes
-  // it into every CTA's receive slots.
-  auto publish = [&](auto slot_c, int64_t dn, int pb) {
-    constexpr int S = decltype(slot_c)::value;
-    K bv = 0;
-    int bg = -1;
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-      const int i = tid + NT * r;
-      const K v = PivKey<T>::of(pr[r][S]);
-      if (i < nloc && base + i >= dn && v > bv) { bv = v; bg = (int)(base + i); }
-    }
-    {
-      int src;
-      warp_pivot_choice(bv, bg, src);
-    }
-    // the stores are issued by the owning warp only (a predicated-off store
-    // still occupies the shared-memory pipe)
-    if (bg >= 0) {
-      const int lw = (int)(bg - base);  // the winner's local row
-#pragma unroll
-      for (int r = 0; r < RPT; ++r)
-        if (lw >= NT * r && lw < NT * (r + 1)) {
-          if (tid + NT * r == lw) row_store<T, W>(s_crowv[pb][warp], pr[r]);
-        }
-    }
-    const int64_t ldn = dn - base;
-    const bool own_diag = ldn >= 0 && ldn < nloc;
-    if (own_diag && (((int)ldn & (NT - 1)) >> 5) == warp) {
-#pragma unroll
-      for (int r = 0; r < RPT; ++r)
-        if (ldn >= NT * r && ldn < NT * (r + 1)) {
-          if (tid + NT * r == ldn) row_store<T, W>(s_diagv[pb], pr[r]);
-        }
-    }
-    if (lane == 0) { s_cval[pb][warp] = bv; s_crow[pb][warp] = bg; }
-    if (warp != kPusher) {
-      named_bar_arrive(2, NT);
-      return;
-    }
-    named_bar_sync(2, NT);  // every warp's candidate and rows are in shared memory
-    K v = lane < NW ? s_cval[pb][lane] : K(0);
-    int g = lane < NW ? s_crow[pb][lane] : -1;
-    int wsrc;
-    warp_pivot_choice(v, g, wsrc);
-    // lane c writes CTA c's receive slots: the candidate, the candidate row
-    // and, from the diagonal row's CTA, the diagonal row (offsets within
-    // one mapped array stay in that CTA's shared memory window)
-    if (lane < G) {
-      const int4 cand = cand_pack<K>(v, g, wsrc);
-      const int4* rsrc = reinterpret_cast<const int4*>(s_crowv[pb][wsrc < 0 ? 0 : wsrc]);
-      const uint32_t rbar = pan_mapa(pan_saddr(&r_bar[pb]), lane);
-      const uint32_t rc = pan_mapa(pan_saddr(&r_cand[pb][cta]), lane);
-      const uint32_t rr = pan_mapa(pan_saddr(&r_row[pb][cta][0]), lane);
-      pan_st_async(rc, cand, rbar);
-#pragma unroll
-      for (int q = 0; q < RB; ++q) pan_st_async(rr + 16u * q, rsrc[q], rbar);
-      if (own_diag) {
-        const int4* dsrc = reinterpret_cast<const int4*>(s_diagv[pb]);
-        const uint32_t rd = pan_mapa(pan_saddr(&r_diag[pb][0]), lane);
-#pragma unroll
-        for (int q = 0; q < RB; ++q) pan_st_async(rd + 16u * q, dsrc[q], rbar);
-      }
-    }
-  };
-
-  publish(std::integral_constant<int, 0>{}, c0, 0);  // column 0: the rows as loaded
-
-  for (int k = 0; k < w; ++k) {
-    const int64_t d = c0 + k;
-    const int buf = k & 1;
-    // 1. warp 0: the winner over the CTAs of the cluster, the pivot row and,
-    //    for the pivot row's CTA, the old diagonal row
-    if (warp == 0) {
-      if (!bad && !pan_bar_wait(pan_saddr(&r_bar[buf]), (uint32_t)(k >> 1) & 1u, err)) bad = true;
-      if (lane == 0 && k + 2 < w) pan_bar_arm(pan_saddr(&r_bar[buf]), rx_bytes);  // column k + 2
-      K v = 0;
-      int g = -1, ew = 0;
-      if (lane < G) cand_unpack<K>(r_cand[buf][lane], v, g, ew);
-      int ec;  // the winning CTA
-      warp_pivot_choice(v, g, ec);
-      const int64_t p = g < 0 ? d : (int64_t)g;  // kp = k when amax == 0
-      // received rows are in the slot order of step k-1: lane j takes slot
-      // j + 1 and finishes its step-(k-1) update (slots 2 .. w-k of step k-1)
-      const int js = k > 0 ? ((lane + 1) & (W - 1)) : lane;
-      T dv = r_diag[buf][js];
-      T pv = p != d ? r_row[buf][ec < 0 ? 0 : ec][js] : dv;
-      if (k > 0) {
-        const T u = s_piv[buf ^ 1][js];
-        const T ld = __shfl_sync(kAll, dv, W - 1);  // slot 0 of step k-1: the multiplier
-        const T lp = __shfl_sync(kAll, pv, W - 1);
-        if (lane >= 1 && lane < w - k) {
-          dv = fma(-ld, u, dv);
-          pv = fma(-lp, u, pv);
-        }
-      }
-      // 1 / |pivot| from warp 1
-      named_bar_sync(1, 64);
-      const T inv_mag = s_rinv[ec < 0 ? 0 : ec];
-      s_piv[buf][lane] = pv;
-      if (p != d && p >= base && p < base + nloc) s_old[lane] = dv;
-      if (lane == 0) {
-        s_p = (int)p;
-        // no candidate: the pivot is the diagonal entry, zero or NaN
-        s_inv = g >= 0 ? with_sign_of(inv_mag, pv) : (PivKey<T>::nonzero(pv) ? T(1) / pv : T(0));
-      }
-    } else if (warp == 1) {
-      // 1 / |candidate| of every received candidate (its key is the bit
-      // pattern of |a|), beside warp 0's reduction: the division is a long
-      // dependent sequence
-      if (!bad && !pan_bar_wait(pan_saddr(&r_bar[buf]), (uint32_t)(k >> 1) & 1u, err)) bad = true;
-      K v = 0;
-      int g = -1, ew = 0;
-      if (lane < G) cand_unpack<K>(r_cand[buf][lane], v, g, ew);
-      const T rinv = T(1) / key_magnitude<T>(g >= 0 ? v : K(1));
-      if (lane < G) s_rinv[lane] = rinv;
-      named_bar_arrive(1, 64);
-    }
-    __syncthreads();
-    const int64_t p = s_p;
-    const T piv = s_piv[buf][0];
-    const bool nz = PivKey<T>::nonzero(piv);
-    if (cta == 0 && tid == 0) {
-      ipiv[d] = p + 1;
-      if (!nz && info_local == 0) info_local = d + 1;
-    }
-    // 2. interchange (nonzero pivot only) and scale
-    const bool swap = nz && p != d;
-    const T inv = s_inv;  // 1 / piv, computed once by warp 0
-    const int lim = w - k;  // slots 1..lim-1 hold columns k+1..w-1
-    T l[RPT];
-    bool upd[RPT];
-    if (swap) {
-      // only the warps holding row d or row p load
-      const int64_t ld = d - base, lp = p - base;
-      const bool own_d = ld >= 0 && ld < nloc && (((int)ld & (NT - 1)) >> 5) == warp;
-      const bool own_p = lp >= 0 && lp < nloc && (((int)lp & (NT - 1)) >> 5) == warp;
-      if (own_d || own_p) {
-#pragma unroll
-        for (int r = 0; r < RPT; ++r) {
-          const int64_t gi = base + tid + NT * r;
-          if (gi == d) row_load<T, W>(pr[r], s_piv[buf]);
-          else if (gi == p) row_load<T, W>(pr[r], s_old);
-        }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-      const int i = tid + NT * r;
-      upd[r] = i < nloc && base + i > d;
-      l[r] = pr[r][0];
-    }
-    if (warp_rows) {
-#pragma unroll
-      for (int r = 0; r < RPT; ++r) {
-        if (upd[r] && nz) l[r] *= inv;
-        if (upd[r]) pr[r][0] = l[r];
-      }
-    }
-    if (k + 1 < w) {
-      // 3. slot 1 first, publish the candidates of column k + 1, then the
-      //    rest of the rank-1 update while the candidates travel
-      if (warp_rows) {
-        const T u1 = s_piv[buf][1];
-#pragma unroll
-        for (int r = 0; r < RPT; ++r)
-          if (upd[r]) pr[r][1] = fma(-l[r], u1, pr[r][1]);
-      }
-      publish(std::integral_constant<int, 1>{}, d + 1, buf ^ 1);
-      if (warp_rows) {
-        if constexpr (sizeof(T) == 4) {
-          // FP32: predicated FMAs over all slots (no branches)
-#pragma unroll
-          for (int q = 0; q < W / VT::N; ++q) {
-            const typename VT::V pv = reinterpret_cast<const typename VT::V*>(s_piv[buf])[q];
-#pragma unroll
-            for (int e = 0; e < VT::N; ++e) {
-              const int j = q * VT::N + e;
-              if (j >= 2 && j < lim) {
-                const T u = VT::get(pv, e);
-#pragma unroll
-                for (int r = 0; r < RPT; ++r)
-                  if (upd[r]) pr[r][j] = fma(-l[r], u, pr[r][j]);
-              }
-            }
-          }
-        } else {
-          // FP64: stop at the last live slot with a uniform branch, so the FP64
-          // pipe only sees the FMAs that do work; the pivot row is read two
-          // slots per 16-byte load
-#pragma unroll
-          for (int j = 2; j < W; j += 2) {
-            if (j >= lim) break;
-            const typename VT::V u2 = reinterpret_cast<const typename VT::V*>(s_piv[buf])[j / 2];
-#pragma unroll
-            for (int r = 0; r < RPT; ++r)
-              if (upd[r]) pr[r][j] = fma(-l[r], VT::get(u2, 0), pr[r][j]);
-            if (j + 1 >= lim) break;
-#pragma unroll
-            for (int r = 0; r < RPT; ++r)
-              if (upd[r]) pr[r][j + 1] = fma(-l[r], VT::get(u2, 1), pr[r][j + 1]);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < RPT; ++r) {
-      const T t0 = pr[r][0];
-#pragma unroll
-      for (int j = 0; j < W - 1; ++j) pr[r][j] = pr[r][j + 1];
-      pr[r][W - 1] = t0;
-    }
-  }
-  // after w steps slot j holds column (w + j) mod 32
-#pragma unroll
-  for (int r = 0; r < RPT; ++r) {
-    const int i = tid + NT * r;
-    if (i < nloc)
-#pragma unroll
-      for (int j = 0; j < W; ++j) {
-        const int c = (w + j) & (W - 1);
-        if (c < w) A[(base + i) + (c0 + c) * lda] = pr[r][j];
-      }
-  }
-  if (cta == 0 && tid == 0 && info_local != 0 && *info_out == 0) *info_out = info_local;
-  cluster.sync();  // no CTA exits while a push to it may be in flight
-}
-
 // ---------------------------------------------------------------------------
 // laswp for one leaf: interchanges ipiv[c0, c0+w) applied to every column
 // outside [c0, c0+w) (blocked_lufact.jl:126-141 applies them to [1, j0) and
@@ -804,6 +418,65 @@ laswp_leaf_kernel(T* __restrict__ A, int64_t lda, int64_t m, int64_t ncols_total
     if (lane + 32 < nmv) a[mv_dst[lane + 32]] = v1;
     if (b2 && lane < nmv) b2[mv_dst[lane]] = u0;
     if (b2 && lane + 32 < nmv) b2[mv_dst[lane + 32]] = u1;
+  }
+}
+
+// The same from composed moves (the sub-panel kernel's output): every warp
+// carries two columns per pass through up to 256 moves, all loads in flight
+// before the stores.
+template <typename T>
+__global__ void __launch_bounds__(256)
+laswp_moves_kernel(T* __restrict__ A, int64_t lda, int64_t ncols_total, int64_t c0, int w,
+                   const LeafMoves* __restrict__ mv, int32_t* __restrict__ perm) {
+  constexpr int MPL = 2 * kLeafMaxW / 32;  // moves per lane, at most
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nmv = mv->count;
+  if (nmv == 0) return;
+  int dst[MPL], src[MPL];
+#pragma unroll
+  for (int i = 0; i < MPL; ++i) {
+    const int e = lane + 32 * i;
+    const int2 x = e < nmv ? mv->mv[e] : make_int2(-1, 0);
+    dst[i] = x.x;
+    src[i] = x.y;
+  }
+  const int nl = (nmv + 31) >> 5;
+  if (perm != nullptr && blockIdx.x == 0 && warp == 0) {
+    // the row permutation (original row of each row) moves like one more column
+    int32_t p[MPL];
+#pragma unroll
+    for (int i = 0; i < MPL; ++i)
+      if (i < nl && dst[i] >= 0) p[i] = perm[src[i]];
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < MPL; ++i)
+      if (i < nl && dst[i] >= 0) perm[dst[i]] = p[i];
+  }
+  const int64_t nother = ncols_total - w;
+  const int64_t stride = (int64_t)gridDim.x * 8;
+  for (int64_t q = (int64_t)blockIdx.x * 8 + warp; q < nother; q += 2 * stride) {
+    const int64_t q2 = q + stride;
+    T* a = A + (q < c0 ? q : q + w) * lda;
+    T* b = q2 < nother ? A + (q2 < c0 ? q2 : q2 + w) * lda : nullptr;
+    T v[MPL], u[MPL];
+#pragma unroll
+    for (int i = 0; i < MPL; ++i) {
+      if (i >= nl) break;
+      v[i] = u[i] = T(0);
+      if (dst[i] >= 0) {
+        v[i] = a[src[i]];
+        if (b) u[i] = b[src[i]];
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < MPL; ++i) {
+      if (i >= nl) break;
+      if (dst[i] >= 0) {
+        a[dst[i]] = v[i];
+        if (b) b[dst[i]] = u[i];
+      }
+    }
   }
 }
 
@@ -1250,7 +923,8 @@ size_t getrf_scratch_bytes(int64_t m, int64_t n, int elem_size, int panel_width,
   size_t b = 256;                     // DevScratch, aligned
   b += 2 * G * elem_size + 2 * G * sizeof(int64_t);
   b += 2 * G * kPanelMaxW * elem_size + 2 * kPanelMaxW * elem_size;
-  return b + 1024;
+  b += sizeof(LeafMoves);
+  return b + 2048;
 }
 
 template <typename T>
@@ -1264,6 +938,7 @@ void getrf_carve(GetrfPlan<T>& p, void* base, size_t bytes, int device) {
   p.slots.cand_row = reinterpret_cast<int64_t*>(take(2 * G * sizeof(int64_t)));
   p.slots.cand_rowvals = reinterpret_cast<T*>(take(2 * G * kPanelMaxW * sizeof(T)));
   p.slots.diag_rowvals = reinterpret_cast<T*>(take(2 * kPanelMaxW * sizeof(T)));
+  p.moves = reinterpret_cast<LeafMoves*>(take(sizeof(LeafMoves)));
   (void)bytes;
 }
 
@@ -1353,72 +1028,16 @@ struct Driver {
     return c == 1;
   }
 
-  template <int RPT>
-  bool panel_reg_launch(int64_t c0, int w, int cs) {
-    const int64_t M = p.m - c0;
-    const int64_t R = (M + cs - 1) / cs;
-    if (R > (int64_t)kRegPanelThreads * RPT || !reg_cluster_ok<RPT>(cs)) return false;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(cs);
-    cfg.blockDim = dim3(kRegPanelThreads);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = cs;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    double fl = 0;
-    for (int k = 0; k < w; ++k) fl += (double)(M - k - 1) * (1.0 + 2.0 * (w - k - 1));
-    LaunchScope ls(K_PANEL, fl, 2.0 * M * w * sizeof(T), s);
-    check(cudaLaunchKernelEx(&cfg, panel_reg_kernel<T, RPT>, p.A, p.lda, p.m, c0, w, p.ipiv, p.info, (int)R,
-                             p.scratch));
-    return true;
+  // Leaf width at row c0: the sub-panel kernel's where it takes the leaf
+  // (0 in sub_width: it does not), else panel_width.
+  int sub_width(int64_t c0) const {
+    if (forced == 1 || forced == 2 || !p.use_sub_panel || !p.moves) return 0;
+    if (std::is_same<T, float>::value && ((p.nopivot && p.tslu_work) || (p.tslu && p.tslu_work && p.m - c0 > 512))) return 0;
+    return panel_sub_width<T>(p.m - c0);
   }
-
-  // Register panel: the rows spread evenly over up to 16 CTAs of one cluster
-  // (at least 128 rows each), one or two rows per thread; false when the
-  // panel is taller or not launchable.
-  bool panel_reg(int64_t c0, int w) {
-    const int64_t M = p.m - c0;
-    // FP64 leaves above 8192 rows (two rows per thread would not fit the
-    // registers) go to the grid kernel
-    if (sizeof(T) == 8 && M > 8192) return false;
-    const int cs = (int)std::min<int64_t>(16, std::max<int64_t>(1, (M + 127) / 128));
-    const int64_t R = (M + cs - 1) / cs;
-    if (R <= kRegPanelThreads) return panel_reg_launch<1>(c0, w, cs);
-    if constexpr (sizeof(T) == 4) {
-      if (R <= 2 * kRegPanelThreads) return panel_reg_launch<2>(c0, w, cs);
-    }
-    return false;
-  }
-
-  template <int RPT>
-  static bool reg_cluster_ok(int cs) {
-    static std::mutex mu;
-    static int cache[17] = {};  // 0 unknown, 1 ok, -1 no (per process and instantiation)
-    std::lock_guard<std::mutex> g(mu);
-    int& c = cache[cs];
-    if (c == 0) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(cs);
-      cfg.blockDim = dim3(kRegPanelThreads);
-      cfg.dynamicSmemBytes = 0;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = cs;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      int nclusters = 0;
-      cudaError_t e = cudaOccupancyMaxActiveClusters(&nclusters, panel_reg_kernel<T, RPT>, &cfg);
-      c = (e == cudaSuccess && nclusters >= 1) ? 1 : -1;
-      cudaGetLastError();
-    }
-    return c == 1;
+  int leaf_width(int64_t c0) const {
+    const int w = sub_width(c0);
+    return w > 0 ? w : p.panel_width;
   }
 
   void panel(int64_t c0, int w) {
@@ -1438,9 +1057,10 @@ struct Driver {
       }
     }
     // forced: 0 automatic, 1 grid kernel only, 2 shared-memory cluster kernel
-    // where it fits, 3 register kernel where it fits (falling back in order)
-    if (forced != 1 && forced != 2 && p.use_reg_panel && panel_reg(c0, w)) {
-      laswp(c0, w);
+    // where it fits, 3 sub-panel kernel where it fits (falling back in order)
+    if (sub_width(c0) >= w) {
+      check(panel_sub_launch<T>(p.A, p.lda, p.m, c0, w, p.ipiv, p.info, p.moves, p.scratch, s));
+      laswp(c0, w, true);
       return;
     }
     if (forced != 1 && p.use_cluster_panel && panel_cluster(c0, w)) {
@@ -1490,7 +1110,8 @@ struct Driver {
   // interchanges of the leaf on every other column
   // The leaf's interchanges on every other column, and on the row permutation
   // (so getrs can gather through it without replaying ipiv).
-  void laswp(int64_t c0, int w) {
+  // composed: by the moves the sub-panel kernel left, else from ipiv.
+  void laswp(int64_t c0, int w, bool composed = false) {
     const DeviceInfo& di = device_info(device);
     const int64_t nother = p.n - w;
     // CTAs per SM (GBLU_LASWP_CTAS_PER_SM overrides): every CTA first turns
@@ -1502,7 +1123,8 @@ struct Driver {
     }();
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((nother + 7) / 8, (int64_t)di.num_sms * per_sm));
     LaunchScope ls(K_LASWP, 0.0, 4.0 * w * std::max<int64_t>(nother, 0) * sizeof(T), s);
-    laswp_leaf_kernel<T><<<blocks, 256, 0, s>>>(p.A, p.lda, p.m, p.n, c0, w, p.ipiv, p.scratch, p.perm);
+    if (composed) laswp_moves_kernel<T><<<blocks, 256, 0, s>>>(p.A, p.lda, p.n, c0, w, p.moves, p.perm);
+    else laswp_leaf_kernel<T><<<blocks, 256, 0, s>>>(p.A, p.lda, p.m, p.n, c0, w, p.ipiv, p.scratch, p.perm);
     check(cudaGetLastError());
   }
 
@@ -1603,7 +1225,7 @@ struct Driver {
   }
 
   void rec(int64_t c0, int64_t w) {
-    const int wb = p.panel_width;
+    const int wb = leaf_width(c0);
     if (w <= wb) {
       panel(c0, (int)w);
       return;
@@ -1655,9 +1277,8 @@ void getrf_configure(int device) {
   cudaFuncSetAttribute(panel_cluster_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
   cudaFuncSetAttribute(panel_cluster_kernel<double>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   cudaFuncSetAttribute(panel_cluster_kernel<float>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  cudaFuncSetAttribute(panel_reg_kernel<double, 1>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  cudaFuncSetAttribute(panel_reg_kernel<float, 1>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  cudaFuncSetAttribute(panel_reg_kernel<float, 2>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  panel_sub_ready<double>();
+  panel_sub_ready<float>();
   cudaFuncSetAttribute(trsm_lunit_kernel<double, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)trsm_smem<double, 128>());
   cudaFuncSetAttribute(trsm_lunit_kernel<float, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1669,7 +1290,7 @@ void getrf_configure(int device) {
   tslu_configure(device);
 }
 
-// GBLU_PANEL=grid|cluster|reg forces one panel kernel (where the panel fits
+// GBLU_PANEL=grid|cluster|reg forces one panel kernel (reg: the sub-panel kernel) (where the panel fits
 // it; the kernels give identical results), so every variant can be tested on
 // small matrices.  Read at each factorization.
 int forced_panel_kind() {

@@ -1,10 +1,12 @@
 // Bitwise check of the library's Markstein division against the IEEE division
 // on random operands (all significands, including the all-ones and power-of-two
-// edge cases, and exponents across the range where the fast path is used).
+// edge cases, and exponents across the range where the fast path is used), and
+// of the sub-panel kernel's integer reciprocal against 1 / x.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "../device_util.cuh"
+#include "../panel.cuh"
 
 namespace {
 __device__ __forceinline__ uint64_t mix64(uint64_t x) {
@@ -61,6 +63,46 @@ extern "C" int32_t gblu_tool_divcheck(int64_t n, uint64_t seed, uint64_t* mism_f
   cudaMemset(d, 0, 2 * sizeof(unsigned long long));
   divcheck_kernel<double, uint64_t><<<1024, 256>>>(seed, n, d);
   divcheck_kernel<float, uint32_t><<<1024, 256>>>(seed ^ 0x5555, n, d + 1);
+  unsigned long long h[2] = {0, 0};
+  cudaError_t e = cudaMemcpy(h, d, sizeof(h), cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  if (e != cudaSuccess) return 2;
+  *mism_f64 = h[0];
+  *mism_f32 = h[1];
+  return 0;
+}
+
+namespace {
+// recip_normal against 1 / x: every FP32 significand at three exponents, and
+// n random FP64 operands (edge significands as above, every exponent it takes).
+__global__ void recipcheck_kernel(uint64_t seed, int64_t n, unsigned long long* bad64, unsigned long long* bad32) {
+  unsigned long long b64 = 0, b32 = 0;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
+    const uint64_t h = mix64(seed ^ (2 * i + 1));
+    uint64_t mant = h & ((1ull << 52) - 1);
+    if ((h >> 60) == 0) mant = (1ull << 52) - 1 - (mant & 7);
+    if ((h >> 60) == 1) mant = mant & 7;
+    const double x = __longlong_as_double((long long)(((1 + (h >> 11) % 2043) << 52) | mant));
+    if (!gblu::recip_in_range(x) ||
+        __double_as_longlong(gblu::recip_normal(x)) != __double_as_longlong(1.0 / x)) ++b64;
+  }
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 3ll << 23; i += stride) {
+    const unsigned e = (i >> 23) == 0 ? 1u : (i >> 23) == 1 ? 127u : 251u;
+    const float x = __uint_as_float((e << 23) | (unsigned)(i & 0x7FFFFF));
+    if (!gblu::recip_in_range(x) || __float_as_uint(gblu::recip_normal(x)) != __float_as_uint(1.0f / x)) ++b32;
+  }
+  if (b64) atomicAdd(bad64, b64);
+  if (b32) atomicAdd(bad32, b32);
+}
+}  // namespace
+
+// Counts the operands whose integer reciprocal differs from 1 / x.
+extern "C" int32_t gblu_tool_recipcheck(int64_t n, uint64_t seed, uint64_t* mism_f64, uint64_t* mism_f32) {
+  unsigned long long* d = nullptr;
+  if (cudaMalloc(&d, 2 * sizeof(unsigned long long)) != cudaSuccess) return 1;
+  cudaMemset(d, 0, 2 * sizeof(unsigned long long));
+  recipcheck_kernel<<<1024, 256>>>(seed, n, d, d + 1);
   unsigned long long h[2] = {0, 0};
   cudaError_t e = cudaMemcpy(h, d, sizeof(h), cudaMemcpyDeviceToHost);
   cudaFree(d);
