@@ -199,6 +199,24 @@ __device__ __forceinline__ void div_markstein_n(T (&a)[N], T b, T y) {
   for (int i = 0; i < N; ++i) a[i] = res[i];
 }
 
+// 2^127 / (2^11 m) within a few units, below 2^64, for a 53-bit significand m
+// (2^52 <= m < 2^53): Newton's iteration on fixed-point words started from the
+// hardware approximation (22 bits -> 43 -> 60).
+__device__ __forceinline__ unsigned long long recip_word(unsigned long long m) {
+  const unsigned long long d = m << 11;             // 2^63 <= d < 2^64
+  const unsigned dh = (unsigned)(d >> 32), dl = (unsigned)d;
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint2float_rz(dh)));
+  // r0 ~ 2^63 / dh, below 2^32
+  const unsigned r0 = (unsigned)min((unsigned long long)__float2ull_rz(y * 9.2233720368547758e18f), 0xFFFFFFFFull);
+  // 2^63 - r0 d / 2^32, about 41 bits, and the first step: R1 ~ 2^127 / d
+  const long long e1 = (long long)((1ull << 63) - ((unsigned long long)r0 * dh + __umulhi(r0, dl)));
+  const unsigned long long R1 =
+      ((unsigned long long)r0 << 32) + (unsigned long long)(((long long)(int)(e1 >> 12) * (long long)(r0 >> 1)) >> 18);
+  const long long e2 = (long long)((1ull << 63) - __umul64hi(R1, d));
+  return R1 + (unsigned long long)(((long long)(int)(e2 >> 1) * (long long)(R1 >> 33)) >> 29);
+}
+
 // IEEE 754 binary64 -> binary32 with round-to-nearest-even, on integer
 // operations only (the FP64 pipe of this GPU retires two lanes per cycle per
 // SM, so a conversion there costs as much as an FP64 FMA).  The standard's

@@ -10,11 +10,17 @@
 // (trans = 'T') is U^T y = b, L^T z = y, x = P^T z as LAPACK dgetrs 'T'.
 //
 // Parallel structure: the matrix is cut into 64-row block rows.  Each CTA takes
-// a block row by ticket (tickets are handed out in launch order, so every CTA
-// waits only for CTAs already running), streams its off-diagonal tiles in
-// order, waiting on a per-block-row flag only right before a tile's
-// solution values are needed, then solves its diagonal block and publishes its
-// rows with a release flag.  All waits are bounded (DEV_TIMEOUT_SOLVE).
+// one block row of one right-hand side by ticket (tickets are handed out in
+// launch order, so every CTA waits only for CTAs already running), streams its
+// off-diagonal tiles in order, polling the published solution values right
+// before a tile needs them, then solves its diagonal block and publishes its
+// rows.  All waits are bounded (DEV_TIMEOUT_SOLVE).
+//
+// A right-hand side a CTA, not several: a warp issues one FP64 instruction per
+// 68 cycles however independent they are, so right-hand sides in one warp add
+// up along the chain.  Five right-hand sides, both sweeps, one CTA per block
+// row for all of them -> one CTA each: exact n = 2000 5.18 -> 0.61 ms,
+// n = 6001 15.5 -> 1.9 ms; fast n = 6001 'N' 3.27 -> 0.82 ms, 'T' 7.55 -> 0.99 ms.
 #include <algorithm>
 
 #include "device_util.cuh"
@@ -28,31 +34,6 @@ constexpr int kTS = kGetrsTile;  // block-row height == tile width
 // fast-solve matrices per 64-row block b, each 64 x 64 column-major:
 // InvL_bb, InvU_bb, InvL_bb L_{b,b-1}, InvU_bb U_{b,b+1}
 constexpr int kInvSlots = 4;
-
-// Wait until flags[j] != 0; returns false on timeout/abort (all threads).
-__device__ __forceinline__ bool wait_flag(const int32_t* flags, int j, DevScratch* scr) {
-  __shared__ int ok;
-  if (threadIdx.x == 0) {
-    int res = 1;
-    unsigned long long t0 = 0;
-    for (unsigned it = 0;; ++it) {
-      if (ld_acquire_i32(flags + j) != 0) break;
-      if (ld_volatile_i32(&scr->error) != 0) { res = 0; break; }
-      if ((it & 63u) == 0) {
-        unsigned long long now = global_ns();
-        if (t0 == 0) t0 = now;
-        else if (now - t0 > kSpinTimeoutNs) {
-          atomicCAS(&scr->error, 0, (int)DEV_TIMEOUT_SOLVE);
-          res = 0;
-          break;
-        }
-      }
-    }
-    ok = res;
-  }
-  __syncthreads();
-  return ok != 0;
-}
 
 constexpr int kSweepThreads = 128;  // all issue copies; threads 0..63 own one row each
 constexpr int kStages = 3;          // tiles in flight per CTA
@@ -107,347 +88,299 @@ __device__ __forceinline__ void issue_tile(T (*t)[tile_ld<T>()], const T* __rest
   }
 }
 
-// One triangular sweep over 64-row block rows.
+// The IEEE division, out of line (inlined, its instructions are scheduled into
+// the chain although the branch to it is not taken).
+template <typename T>
+__device__ __noinline__ T divide_ieee(T a, T b) { return a / b; }
+
+// One lane's store without a branch (a divergent one costs the warp 50 cycles
+// of the chain).
+__device__ __forceinline__ void store_if(bool on, double* p, double v) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %0, 0;\n\t@q st.global.f64 [%1], %2;\n\t}" ::"r"((int)on), "l"(p), "d"(v) : "memory");
+}
+__device__ __forceinline__ void store_if(bool on, float* p, float v) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %0, 0;\n\t@q st.global.f32 [%1], %2;\n\t}" ::"r"((int)on), "l"(p), "f"(v) : "memory");
+}
+__device__ __forceinline__ void store_shared_if(bool on, double* p, double v) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %0, 0;\n\t@q st.volatile.shared.f64 [%1], %2;\n\t}" ::"r"((int)on), "r"((unsigned)__cvta_generic_to_shared(p)), "d"(v) : "memory");
+}
+__device__ __forceinline__ void store_shared_if(bool on, float* p, float v) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %0, 0;\n\t@q st.volatile.shared.f32 [%1], %2;\n\t}" ::"r"((int)on), "r"((unsigned)__cvta_generic_to_shared(p)), "f"(v) : "memory");
+}
+
+// A value another warp of the CTA leaves in shared memory (the sentinel until
+// then).  Bounded like every wait; zero once any CTA failed.
+template <typename T>
+__device__ __forceinline__ T smem_value(const T* p, DevScratch* scr) {
+  using U = typename SweepBits<T>::U;
+  const volatile U* q = reinterpret_cast<const volatile U*>(p);
+  unsigned long long t0 = 0;
+  for (unsigned it = 0;; ++it) {
+    const U v = *q;
+    if (v != SweepBits<T>::kSentinel) return SweepBits<T>::as_t(v);
+    if ((it & 1023u) == 1023u) {
+      if (ld_volatile_i32(&scr->error) != 0) return T(0);
+      const unsigned long long now = global_ns();
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > kSpinTimeoutNs) {
+        atomicCAS(&scr->error, 0, (int)DEV_TIMEOUT_SOLVE);
+        return T(0);
+      }
+    }
+  }
+}
+
+// One exact triangular sweep over 64-row block rows, one right-hand side per CTA.
 //   FWD  : block rows first-to-last, columns ascending; 'N' unit-lower L with
 //          the right-hand side gathered through perm, 'T' non-unit U^T.
 //   !FWD : block rows last-to-first, columns descending; 'N' non-unit U,
-//          'T' unit L^T; results also scattered to Out (through perm for 'T').
-// Each row accumulates its updates in exactly the reference's order; the
-// diagonal block is solved by warp shuffles (no block barrier per column).
+//          'T' unit L^T; results scattered to Out (through perm for 'T').
+// Each row accumulates its updates in exactly the reference's order.  Warps 0
+// and 1 own the block's 32-row halves (a row a lane); warps 2 and 3 help with
+// the copies and poll the values of the block row just before this one, which
+// the row warps apply one by one as they arrive (published as soon as final).
+// Then the first half's 32-step chain, its coefficients in registers, the
+// second half applying the first's solutions as they come, and its chain.
 //
-// FAST: the same wavefront without the reference's order: each row keeps
-// four independent partial sums over the off-diagonal tiles, and the
-// diagonal block is applied as a 64 x 64 matrix-vector product with its
-// precomputed inverse (inv: [block][L, U][64 x 64], column-major), so a block
-// row's critical path is two short product chains instead of 64 dependent
-// division / FMA steps.  Backward-error accurate, not bit-exact.
-template <typename T, int NR, bool TRANS, bool FWD, bool FAST>
+// Bound: the chain of n dependent steps, each a shuffle and an FP64
+// instruction (35 + 68 cycles), and three more of those for the division by a
+// non-unit diagonal entry.  In place: 123 cycles a step (unit) and 425
+// (non-unit), against 203 and 500 when a step waited for a shared-memory load
+// of its coefficient and for a branch to publish; n = 2000, one right-hand
+// side, both sweeps: 0.76 -> 0.61 ms.
+template <typename T, bool TRANS, bool FWD>
 __global__ void __launch_bounds__(kSweepThreads)
 solve_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32_t* __restrict__ perm,
                    const T* __restrict__ In, int64_t ldi, T* __restrict__ Y, int64_t ldy,
-                   T* __restrict__ Out, int64_t ldo, int nrhs, int32_t* __restrict__ flags,
-                   DevScratch* __restrict__ scr, const T* __restrict__ inv) {
+                   T* __restrict__ Out, int64_t ldo, int nrhs, DevScratch* __restrict__ scr) {
+  using SB = SweepBits<T>;
+  using UB = typename SB::U;
+  constexpr unsigned kAll = 0xffffffffu;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T(*tiles)[kTS][tile_ld<T>()] = reinterpret_cast<T(*)[kTS][tile_ld<T>()]>(smem_raw);
   // 16-byte copies need a 16-byte-aligned matrix and column stride
   const bool vec16 = ((reinterpret_cast<uintptr_t>(LU) | (uintptr_t)(lda * (int64_t)sizeof(T))) & 15) == 0;
-  __shared__ T sx[kTS][NR];
-  __shared__ int s_blk;
-  __shared__ int s_fail;
+  __shared__ T sx[kTS];   // solution values of the current off-diagonal tile
+  __shared__ T s_lx[kTS]; // of the last one, as they arrive (sentinel until then)
+  __shared__ T s_dx[kTS]; // the first half's own solutions, as they become final
+  __shared__ int s_ticket;
   constexpr bool kUnit = FWD != TRANS;  // fwd 'N' (L) and bwd 'T' (L^T) have unit diagonals
-  // FP64: rows are published as soon as they are final and the next block
-  // row applies them as they come (its last tile is 64 dependent 64-cycle
-  // FMAs per row); FP32 tiles are cheap, so rows are published at the end.
-  constexpr bool kEarly = sizeof(T) == 8 && !FAST;
   const int nblk = (int)((n + kTS - 1) / kTS);
-  if (threadIdx.x == 0) {
-    const int t = (int)atomicAdd(&scr->ticket, 1u);
-    s_blk = FWD ? t : nblk - 1 - t;
-    s_fail = 0;
-  }
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) s_ticket = (int)atomicAdd(&scr->ticket, 1u);
+  if (tid < kTS) s_lx[tid] = s_dx[tid] = SB::as_t(SB::kSentinel);
   __syncthreads();
-  const int blk = s_blk;
+  const int ord = s_ticket / nrhs, rhs = s_ticket - ord * nrhs;
+  const int blk = FWD ? ord : nblk - 1 - ord;
+  if (In) In += rhs * ldi;
+  Y += rhs * ldy;
+  if (Out) Out += rhs * ldo;
   const int64_t r0 = (int64_t)blk * kTS;
   const int nr = (int)min((int64_t)kTS, n - r0);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int r = tid;  // row within the block (threads 0..63)
   const bool valid = r < nr;
-  T acc[NR];
-#pragma unroll
-  for (int q = 0; q < NR; ++q) {
-    acc[q] = T(0);
-    if (valid && q < nrhs) {
-      if (FWD) acc[q] = In[(TRANS ? r0 + r : (int64_t)perm[r0 + r]) + q * ldi];
-      else acc[q] = Y[(r0 + r) + q * ldy];
-    }
+  T acc = T(0);
+  T* dst = nullptr;   // where this row's solution is published
+  if (valid) {
+    const int64_t prow = (FWD != TRANS) ? (int64_t)perm[r0 + r] : r0 + r;
+    // NaN canonical from here on (arithmetic gives no other), so no published
+    // value is the sentinel
+    acc = SB::canon(FWD ? In[TRANS ? r0 + r : prow] : Y[r0 + r]);
+    dst = FWD ? Y + r0 + r : Out + (TRANS ? prow : r0 + r);
   }
   const int noff = FWD ? blk : nblk - 1 - blk;  // off-diagonal tiles of this block row
   const int ntiles = noff + 1;                  // + the diagonal tile
   auto col_block = [&](int t) -> int { return t < noff ? (FWD ? t : nblk - 1 - t) : blk; };
   auto issue = [&](int t) {
-    if (FAST && t == noff) {  // op(inverse of the diagonal block): tile[c][r] = op(Inv)(r, c)
-      const T* ib = inv + ((int64_t)blk * kInvSlots + (kUnit ? 0 : 1)) * (kTS * kTS);
-      issue_tile<T, TRANS>(tiles[t % kStages], ib, kTS, 0, 0, nr, nr, true);
-      return;
-    }
-    const int cb = col_block(t);
-    const int64_t c0 = (int64_t)cb * kTS;
-    const int nc = (int)min((int64_t)kTS, n - c0);
-    issue_tile<T, TRANS>(tiles[t % kStages], LU, lda, r0, c0, nr, nc, vec16);
+    const int64_t c0 = (int64_t)col_block(t) * kTS;
+    issue_tile<T, TRANS>(tiles[t % kStages], LU, lda, r0, c0, nr, (int)min((int64_t)kTS, n - c0), vec16);
   };
-  // FAST: three more partial sums per right-hand side (acc is the first)
-  T acc2[FAST ? 3 : 1][NR];
-#pragma unroll
-  for (int j = 0; j < (FAST ? 3 : 1); ++j)
-#pragma unroll
-    for (int q = 0; q < NR; ++q) acc2[j][q] = T(0);
 #pragma unroll
   for (int t = 0; t < kStages - 1; ++t) {
     if (t < ntiles) issue(t);
     cp_async_commit();
   }
+  auto src_of = [&](int cb, int c) -> const T* {
+    const int64_t c0 = (int64_t)cb * kTS;
+    return FWD ? &Y[c0 + c] : &Out[TRANS ? (int64_t)perm[c0 + c] : c0 + c];
+  };
   // Solution values of the next off-diagonal tile are fetched one tile ahead
   // (most are published long before they are needed); a value still equal to
   // the sentinel is polled until it arrives.
-  using UB = typename SweepBits<T>::U;
-  constexpr int KP = (kTS * NR + kSweepThreads - 1) / kSweepThreads;
-  UB pre[KP];
-  auto src_of = [&](int cb, int c, int q) -> const T* {
-    const int64_t c0 = (int64_t)cb * kTS;
-    return FWD ? &Y[(c0 + c) + q * ldy] : &Out[(TRANS ? (int64_t)perm[c0 + c] : c0 + c) + q * ldo];
-  };
+  UB pre = 0;
   auto prefetch = [&](int t) {
     const int cb = col_block(t);
     const int nc = (int)min((int64_t)kTS, n - (int64_t)cb * kTS);
-#pragma unroll
-    for (int k = 0; k < KP; ++k) {
-      const int idx = tid + k * kSweepThreads;
-      const int c = idx / NR, q = idx - c * NR;
-      pre[k] = (idx < kTS * NR && q < nrhs && c < nc) ? SweepBits<T>::load(src_of(cb, c, q)) : UB(0);
-    }
+    if (tid < nc) pre = SB::load(src_of(cb, tid));
   };
-  // (FP64: the last off-diagonal tile is consumed as it is published)
-  if (noff > (kEarly ? 1 : 0)) prefetch(0);
-  // this row's solution values, to the sweep's output (dependents poll them)
-  auto publish_row = [&]() {
-#pragma unroll
-    for (int q = 0; q < NR; ++q)
-      if (q < nrhs) {
-        const T v = SweepBits<T>::canon(acc[q]);
-        if (FWD) Y[(r0 + r) + q * ldy] = v;
-        else Out[(TRANS ? (int64_t)perm[r0 + r] : r0 + r) + q * ldo] = v;
-      }
-  };
-  for (int t = 0; t < ntiles; ++t) {
+  if (noff > 1) prefetch(0);
+  for (int t = 0; t < noff - 1; ++t) {
+    cp_async_wait<kStages - 2>();  // tile t has landed
+    __syncthreads();               // everywhere, and the slot of tile t - 1 is free
     if (t + kStages - 1 < ntiles) issue(t + kStages - 1);
     cp_async_commit();
-    cp_async_wait<kStages - 1>();
-    __syncthreads();
     T(*tile)[tile_ld<T>()] = tiles[t % kStages];
-    if (kEarly && t == noff - 1) {
-      // The tile of the block row just before this one in the sweep: its
-      // rows are published one by one while that block solves its diagonal,
-      // so it is applied CH columns at a time in sweep order, warp 2 polling
-      // the next columns while warps 0-1 apply the previous ones.
-      const int cb = col_block(t);
-      const int nc = (int)min((int64_t)kTS, n - (int64_t)cb * kTS);
-      constexpr int CH = 8, NCH = kTS / CH;
-      for (int ch = 0; ch <= NCH; ++ch) {
-        if (warp == 2 && ch < NCH) {
-          const int cbeg = FWD ? CH * ch : kTS - CH * (ch + 1);
-          for (int idx = lane; idx < CH * NR; idx += 32) {
-            const int c = cbeg + idx / NR, q = idx % NR;
-            T v = T(0);
-            if (q < nrhs && c < nc && !poll_value(src_of(cb, c, q), scr, &v)) s_fail = 1;
-            sx[c][q] = v;
-          }
-        }
-        if (warp < 3) named_bar_sync(1, 96);
-        if (ch > 0 && tid < kTS) {
-          const int pc = ch - 1;
-          if (FWD) {
-#pragma unroll
-            for (int c = CH * pc; c < CH * pc + CH; ++c) {
-              const T l = tile[c][r];
-#pragma unroll
-              for (int q = 0; q < NR; ++q) acc[q] = fma(-l, sx[c][q], acc[q]);
-            }
-          } else {
-#pragma unroll
-            for (int c = kTS - CH * pc - 1; c >= kTS - CH * (pc + 1); --c) {
-              if (c >= nc) continue;
-              const T u = tile[c][r];
-#pragma unroll
-              for (int q = 0; q < NR; ++q) acc[q] = fma(-u, sx[c][q], acc[q]);
-            }
-          }
-        }
+    const int cb = col_block(t);
+    const int nc = (int)min((int64_t)kTS, n - (int64_t)cb * kTS);
+    int ok = 1;
+    if (tid < kTS) {
+      T v = T(0);
+      if (tid < nc) {
+        if (pre != SB::kSentinel) v = SB::as_t(pre);
+        else if (!poll_value(src_of(cb, tid), scr, &v)) ok = 0;
       }
-      if (!__syncthreads_and(s_fail == 0)) {
-        cp_async_wait<0>();  // no copy may land after the CTA has left
-        return;
-      }
-      continue;
+      sx[tid] = v;
     }
-    if (t < noff) {
-      const int cb = col_block(t);
-      const int64_t c0 = (int64_t)cb * kTS;
-      const int nc = (int)min((int64_t)kTS, n - c0);
-      int ok = 1;
-#pragma unroll
-      for (int k = 0; k < KP; ++k) {
-        const int idx = tid + k * kSweepThreads;
-        if (idx >= kTS * NR) continue;
-        const int c = idx / NR, q = idx - c * NR;
-        T v = T(0);
-        if (q < nrhs && c < nc) {
-          if (pre[k] != SweepBits<T>::kSentinel) v = SweepBits<T>::as_t(pre[k]);
-          else if (!poll_value(src_of(cb, c, q), scr, &v)) ok = 0;
-        }
-        sx[c][q] = v;
-      }
-      if (!__syncthreads_and(ok)) {
-        cp_async_wait<0>();  // no copy may land after the CTA has left
-        return;
-      }
-      if (t + 1 < noff - (kEarly ? 1 : 0)) prefetch(t + 1);
-      if constexpr (FAST) {
-        // four independent partial sums (columns c = 4i + j); entries past nc
-        // are zero in both the tile and sx
-        if (tid < kTS) {
-#pragma unroll 4
-          for (int c = 0; c < kTS; c += 4) {
-            const T l0 = tile[c][r], l1 = tile[c + 1][r], l2 = tile[c + 2][r], l3 = tile[c + 3][r];
-#pragma unroll
-            for (int q = 0; q < NR; ++q) {
-              acc[q] = fma(-l0, sx[c][q], acc[q]);
-              acc2[0][q] = fma(-l1, sx[c + 1][q], acc2[0][q]);
-              acc2[1][q] = fma(-l2, sx[c + 2][q], acc2[1][q]);
-              acc2[2][q] = fma(-l3, sx[c + 3][q], acc2[2][q]);
-            }
-          }
-        }
-      } else if (tid < kTS) {
-        if (FWD) {
-#pragma unroll 8
-          for (int c = 0; c < kTS; ++c) {
-            const T l = tile[c][r];
-#pragma unroll
-            for (int q = 0; q < NR; ++q) acc[q] = fma(-l, sx[c][q], acc[q]);
-          }
-        } else if (nc == kTS) {
-#pragma unroll 8
-          for (int c = kTS - 1; c >= 0; --c) {
-            const T u = tile[c][r];
-#pragma unroll
-            for (int q = 0; q < NR; ++q) acc[q] = fma(-u, sx[c][q], acc[q]);
-          }
-        } else {
-          for (int c = nc - 1; c >= 0; --c) {
-            const T u = tile[c][r];
-#pragma unroll
-            for (int q = 0; q < NR; ++q) acc[q] = fma(-u, sx[c][q], acc[q]);
-          }
-        }
-      }
-      __syncthreads();
-      continue;
+    if (!__syncthreads_and(ok)) {
+      cp_async_wait<0>();  // no copy may land after the CTA has left
+      return;
     }
-    if constexpr (FAST) {
-      // ---- diagonal block: x = op(Inv) (b - off-diagonal products) ----
-      if (tid < kTS) {
-#pragma unroll
-        for (int q = 0; q < NR; ++q) {
-          const T tot = (acc[q] + acc2[0][q]) + (acc2[1][q] + acc2[2][q]);
-          sx[r][q] = valid ? tot : T(0);
-        }
-      }
-      __syncthreads();
-      if (tid < kTS) {
-        T y[4][NR];
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-          for (int q = 0; q < NR; ++q) y[j][q] = T(0);
-#pragma unroll 4
-        for (int c = 0; c < kTS; c += 4) {
-          const T m0 = tile[c][r], m1 = tile[c + 1][r], m2 = tile[c + 2][r], m3 = tile[c + 3][r];
-#pragma unroll
-          for (int q = 0; q < NR; ++q) {
-            y[0][q] = fma(m0, sx[c][q], y[0][q]);
-            y[1][q] = fma(m1, sx[c + 1][q], y[1][q]);
-            y[2][q] = fma(m2, sx[c + 2][q], y[2][q]);
-            y[3][q] = fma(m3, sx[c + 3][q], y[3][q]);
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < NR; ++q) acc[q] = (y[0][q] + y[1][q]) + (y[2][q] + y[3][q]);
-      }
-      continue;
-    }
-    // ---- diagonal block: warp shuffles within each 32-row half ----
-
-    // reciprocal of this row's diagonal entry, off the dependency chain
-    const T yrow = (!kUnit && valid && tid < kTS) ? T(1) / tile[r][r] : T(1);
-    const int w_first = FWD ? 0 : 1, w_second = FWD ? 1 : 0;
-    const int lo_second = FWD ? 32 : 0;  // first row of the second half
-    (void)lo_second;
-    // One column of the diagonal chain for all NR right-hand sides: the
-    // divisions (lane `src` only, non-unit diagonal), then the broadcasts,
-    // then the updates, so the NR chains overlap.
-    // keep: the owner also leaves its value in sx for the other warp
-    auto chain_step = [&](int c, int src, bool divide_here, bool update, bool keep) {
-      if (!kUnit && divide_here) {
-        if constexpr (NR == 1) acc[0] = div_markstein(acc[0], tile[c][c], yrow);
-        else div_markstein_n<T, NR>(acc, tile[c][c], yrow);
-      }
-      T xc[NR];
-#pragma unroll
-      for (int q = 0; q < NR; ++q) xc[q] = __shfl_sync(0xffffffffu, acc[q], src);
-      // row c is final: its dependents may start on it (stored while the
-      // broadcast is in flight)
-      if (kEarly && r == c && valid) {
-        publish_row();
-        if (keep)
-#pragma unroll
-          for (int q = 0; q < NR; ++q) sx[c][q] = acc[q];
-      }
-      if (update) {
-        const T a = tile[c][r];
-#pragma unroll
-        for (int q = 0; q < NR; ++q) acc[q] = fma(-a, xc[q], acc[q]);
-      }
-    };
-    // FP64: the second warp applies the first half's solutions eight
-    // columns at a time while the first warp is still solving (one named
-    // barrier per group of eight), instead of re-applying all of them as a
-    // chain of 64-cycle FMAs afterwards.
-    const bool prog = kEarly && nr > 32;
-    const int m1 = FWD ? min(nr, 32) : nr - 32;  // columns of the first half
-    if (warp == w_first) {
-      // columns of the first half, in sweep order
-      for (int st = 0; st < m1; ++st) {
-        const int c = FWD ? st : nr - 1 - st;
-        if (FWD) chain_step(c, c, lane == c, r > c && r < nr, prog);
-        else chain_step(c, c - 32, r == c, r < c, prog);
-        if (prog && ((st & 7) == 7 || st == m1 - 1)) named_bar_arrive(2 + (st >> 3), 64);
-      }
-      if (!prog && valid)
-#pragma unroll
-        for (int q = 0; q < NR; ++q) sx[r][q] = acc[q];
-    }
-    if (!prog) __syncthreads();
-    if (warp == w_second) {
-      // the first half's columns applied in sweep order, then this half's chain
-      for (int st = 0; st < m1; ++st) {
-        if (prog && (st & 7) == 0) named_bar_sync(2 + (st >> 3), 64);
-        const int c = FWD ? st : nr - 1 - st;
-        if (FWD && nr <= 32) break;
-#pragma unroll
-        for (int q = 0; q < NR; ++q) acc[q] = fma(-tile[c][r], sx[c][q], acc[q]);
-      }
+    if (t + 1 < noff - 1) prefetch(t + 1);
+    if (tid < kTS) {
       if (FWD) {
-        for (int c = 32; c < nr; ++c) chain_step(c, c - 32, r == c, r > c && r < nr, false);
+#pragma unroll 8
+        for (int c = 0; c < kTS; ++c) acc = fma(-tile[c][r], sx[c], acc);
+      } else if (nc == kTS) {
+#pragma unroll 8
+        for (int c = kTS - 1; c >= 0; --c) acc = fma(-tile[c][r], sx[c], acc);
       } else {
-        for (int c = min(nr, 32) - 1; c >= 0; --c) chain_step(c, c, lane == c, r < c, false);
+        for (int c = nc - 1; c >= 0; --c) acc = fma(-tile[c][r], sx[c], acc);
       }
     }
   }
-  cp_async_wait<0>();
-  if (!kEarly && valid && tid < kTS) publish_row();
-  (void)flags;
+  cp_async_wait<0>();  // the last off-diagonal tile and the diagonal one
+  __syncthreads();
+  if (warp >= 2) {
+    if (noff > 0) {
+      const int cb = col_block(noff - 1);
+      const int nc = (int)min((int64_t)kTS, n - (int64_t)cb * kTS);
+      const int c = tid - 64;
+      const T* p = src_of(cb, c < nc ? c : 0);
+      bool pend = c < nc;
+      unsigned long long t0 = 0;
+      for (unsigned it = 0; __any_sync(kAll, pend); ++it) {
+        if (pend) {
+          const UB v = SB::load(p);
+          if (v != SB::kSentinel) {
+            *reinterpret_cast<volatile UB*>(&s_lx[c]) = v;
+            pend = false;
+          }
+        }
+        if ((it & 63u) == 63u) {
+          bool give_up = ld_volatile_i32(&scr->error) != 0;
+          const unsigned long long now = global_ns();
+          if (t0 == 0) t0 = now;
+          else if (now - t0 > kSpinTimeoutNs) {
+            atomicCAS(&scr->error, 0, (int)DEV_TIMEOUT_SOLVE);
+            give_up = true;
+          }
+          if (give_up) break;  // the row warps see the error word
+        }
+      }
+    }
+    return;
+  }
+  // The row warps.  Coefficients of the own half's diagonal block in registers.
+  T(*dt)[tile_ld<T>()] = tiles[noff % kStages];
+  T a[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) a[i] = dt[32 * warp + i][r];
+  const T dg = (!kUnit && valid) ? dt[r][r] : T(1);
+  const T y = T(1) / dg;
+  const bool y_ok = DivRange<T>::in_range(y);
+  if (noff > 0) {
+    T(*tile)[tile_ld<T>()] = tiles[(noff - 1) % kStages];
+    if (FWD) {
+#pragma unroll 4
+      for (int c = 0; c < kTS; ++c) acc = fma(-tile[c][r], smem_value(&s_lx[c], scr), acc);
+    } else {
+      const int nc = (int)min((int64_t)kTS, n - (int64_t)col_block(noff - 1) * kTS);
+      if (nc == kTS) {
+#pragma unroll 4
+        for (int c = kTS - 1; c >= 0; --c) acc = fma(-tile[c][r], smem_value(&s_lx[c], scr), acc);
+      } else {
+        for (int c = nc - 1; c >= 0; --c) acc = fma(-tile[c][r], smem_value(&s_lx[c], scr), acc);
+      }
+    }
+  }
+  const bool first = warp == (FWD ? 0 : 1);
+  if (!first) {  // the first half's columns, in sweep order
+    if (FWD) {
+      if (nr > 32)
+#pragma unroll 4
+        for (int c = 0; c < 32; ++c) acc = fma(-dt[c][r], smem_value(&s_dx[c], scr), acc);
+    } else {
+      for (int c = nr - 1; c >= 32; --c) acc = fma(-dt[c][r], smem_value(&s_dx[c], scr), acc);
+    }
+  }
+  // The chain: in each step the owner's value is final, goes to every lane, is
+  // published, and updates the rows after it.  The finished rows' registers are
+  // updated too and not used again, so nothing is predicated.
+  if constexpr (kUnit) {
+#pragma unroll
+    for (int st = 0; st < 32; ++st) {
+      const int i = FWD ? st : 31 - st;
+      const int c = 32 * warp + i;
+      if (c >= nr) continue;  // uniform
+      const T x = __shfl_sync(kAll, acc, i);
+      acc = fma(-a[i], x, acc);
+      store_if(lane == i, dst, x);
+      if (first) store_shared_if(lane == i, &s_dx[c], x);
+    }
+  } else {
+    // First divided by the diagonal entry (Markstein's division, every lane by
+    // its own).  Where Markstein's quotient may not be the correctly rounded
+    // one the IEEE division is taken; the branch to it costs 120 cycles of the
+    // chain, so it is tested once per four columns, which then start over.
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+      const T before = acc;
+      T own = T(0);
+      int ok = 1;
+#pragma unroll
+      for (int st = 4 * g; st < 4 * g + 4; ++st) {
+        const int i = FWD ? st : 31 - st;
+        if (32 * warp + i >= nr) continue;  // uniform
+        const T q = acc * y;
+        const T e = fma(-dg, q, acc);
+        const T d = fma(e, y, q);
+        const bool zero = !PivKey<T>::nonzero(acc);  // q is the signed zero
+        const T x = __shfl_sync(kAll, zero ? q : d, i);
+        ok &= __shfl_sync(kAll, (int)(y_ok && (zero || DivRange<T>::in_range(q))), i);
+        own = lane == i ? x : own;
+        acc = fma(-a[i], x, acc);
+      }
+      if (!ok) {
+        acc = before;
+#pragma unroll 1
+        for (int st = 4 * g; st < 4 * g + 4; ++st) {
+          const int i = FWD ? st : 31 - st;
+          if (32 * warp + i >= nr) continue;
+          const T x = __shfl_sync(kAll, divide_ieee(acc, dg), i);
+          own = lane == i ? x : own;
+          acc = fma(-dt[32 * warp + i][r], x, acc);
+        }
+      }
+      const bool mine = (FWD ? lane : 31 - lane) / 4 == g && valid;
+      store_if(mine, dst, own);
+      if (first) store_shared_if(mine, &s_dx[r], own);
+    }
+  }
 }
 
-// Fast 'N' sweeps.  Block row i's solution is x_i = d_i - M_i x_p, where x_p
+// Fast sweeps.  'N': block row i's solution is x_i = d_i - M_i x_p, where x_p
 // is the block row just before it in the sweep, M_i its coupling (fold_kernel)
 // and d_i = Inv_ii (b_i - the products with every earlier block row but x_p):
 // d_i is computed while x_p is still being solved, so only the 64 x 64
-// product M_i x_p lies on the wavefront's critical path.  Two threads per
+// product M_i x_p lies on the wavefront's critical path.  'T' has no coupling:
+// x_i = op(Inv_ii) (b_i - every product).  Two threads per
 // row, each taking half of every tile's columns with four independent
 // partial sums, combined through shared memory.  Tile order per block row:
-// the earlier off-diagonal blocks but the last (in sweep order), Inv_ii,
-// then M_i.  Backward-error accurate, not bit-exact.
-template <typename T, int NR, bool FWD>
+// the earlier off-diagonal blocks (but the last, in sweep order, for 'N'),
+// Inv_ii, then M_i.  NR right-hand sides per CTA: one in FP64 (a warp issues
+// an FP64 instruction per 68 cycles, so more would add up along the chain),
+// up to eight in FP32.  Backward-error accurate, not bit-exact.
+template <typename T, int NR, bool TRANS, bool FWD>
 __global__ void __launch_bounds__(kSweepThreads)
 fast_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32_t* __restrict__ perm,
                   const T* __restrict__ In, int64_t ldi, T* __restrict__ Y, int64_t ldy,
@@ -457,33 +390,38 @@ fast_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32_
   T(*tiles)[kTS][tile_ld<T>()] = reinterpret_cast<T(*)[kTS][tile_ld<T>()]>(smem_raw);
   __shared__ T sx[kTS][NR];
   __shared__ T part[2][kTS][NR];
-  __shared__ int s_blk;
+  __shared__ int s_ticket;
   const bool vec16 = ((reinterpret_cast<uintptr_t>(LU) | (uintptr_t)(lda * (int64_t)sizeof(T))) & 15) == 0;
   const int nblk = (int)((n + kTS - 1) / kTS);
-  if (threadIdx.x == 0) {
-    const int t = (int)atomicAdd(&scr->ticket, 1u);
-    s_blk = FWD ? t : nblk - 1 - t;
-  }
+  constexpr bool kCouple = !TRANS;
+  constexpr bool kUnit = FWD != TRANS;
+  if (threadIdx.x == 0) s_ticket = (int)atomicAdd(&scr->ticket, 1u);
   __syncthreads();
-  const int blk = s_blk;
+  const int groups = (nrhs + NR - 1) / NR;  // CTAs per block row
+  const int ord = s_ticket / groups, q0 = (s_ticket - ord * groups) * NR;
+  const int blk = FWD ? ord : nblk - 1 - ord;
+  nrhs = min(NR, nrhs - q0);
+  if (In) In += q0 * ldi;
+  Y += q0 * ldy;
+  if (Out) Out += q0 * ldo;
   const int64_t r0 = (int64_t)blk * kTS;
   const int nr = (int)min((int64_t)kTS, n - r0);
   const int tid = threadIdx.x, r = tid & 63, h = tid >> 6;
   const bool valid = r < nr;
   const int noff = FWD ? blk : nblk - 1 - blk;  // block rows before this one in the sweep
-  const int nlead = noff > 0 ? noff - 1 : 0;    // off-diagonal tiles before the coupling
-  const int ntiles = nlead + 1 + (noff > 0 ? 1 : 0);
+  const int nlead = kCouple ? max(noff - 1, 0) : noff;  // off-diagonal tiles before the coupling
+  const int ntiles = nlead + 1 + (kCouple && noff > 0 ? 1 : 0);
   const int pcb = FWD ? blk - 1 : blk + 1;      // the coupled block row (noff > 0)
   const int pnc = noff > 0 ? (int)min((int64_t)kTS, n - (int64_t)pcb * kTS) : 0;
   auto col_block = [&](int t) -> int { return FWD ? t : nblk - 1 - t; };
   auto issue = [&](int t) {
     if (t < nlead) {
       const int64_t c0 = (int64_t)col_block(t) * kTS;
-      issue_tile<T, false>(tiles[t % kStages], LU, lda, r0, c0, nr, (int)min((int64_t)kTS, n - c0), vec16);
+      issue_tile<T, TRANS>(tiles[t % kStages], LU, lda, r0, c0, nr, (int)min((int64_t)kTS, n - c0), vec16);
     } else {
       const bool coupling = t > nlead;
-      const int slot = (coupling ? 2 : 0) + (FWD ? 0 : 1);
-      issue_tile<T, false>(tiles[t % kStages], inv + ((int64_t)blk * kInvSlots + slot) * (kTS * kTS), kTS, 0, 0,
+      const int slot = (coupling ? 2 : 0) + (kUnit ? 0 : 1);  // L's, U's
+      issue_tile<T, TRANS>(tiles[t % kStages], inv + ((int64_t)blk * kInvSlots + slot) * (kTS * kTS), kTS, 0, 0,
                            nr, coupling ? pnc : nr, true);
     }
   };
@@ -495,7 +433,7 @@ fast_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32_
   if (h == 0 && valid)
 #pragma unroll
     for (int q = 0; q < NR; ++q)
-      if (q < nrhs) a[0][q] = FWD ? In[(int64_t)perm[r0 + r] + q * ldi] : Y[(r0 + r) + q * ldy];
+      if (q < nrhs) a[0][q] = FWD ? In[(TRANS ? r0 + r : (int64_t)perm[r0 + r]) + q * ldi] : Y[(r0 + r) + q * ldy];
   T d[NR];
 #pragma unroll
   for (int q = 0; q < NR; ++q) d[q] = T(0);
@@ -510,7 +448,7 @@ fast_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32_
   UB pre[KP];
   auto src_of = [&](int cb, int c, int q) -> const T* {
     const int64_t c0 = (int64_t)cb * kTS;
-    return FWD ? &Y[(c0 + c) + q * ldy] : &Out[(c0 + c) + q * ldo];
+    return FWD ? &Y[(c0 + c) + q * ldy] : &Out[(TRANS ? (int64_t)perm[c0 + c] : c0 + c) + q * ldo];
   };
   auto prefetch = [&](int cb) {
     const int nc = (int)min((int64_t)kTS, n - (int64_t)cb * kTS);
@@ -555,12 +493,12 @@ fast_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32_
     }
   };
   if (nlead > 0) prefetch(col_block(0));
-  else if (noff > 0) prefetch(pcb);
+  else if (kCouple && noff > 0) prefetch(pcb);
   for (int t = 0; t < ntiles; ++t) {
+    cp_async_wait<kStages - 2>();  // tile t has landed
+    __syncthreads();               // everywhere, and the slot of tile t - 1 is free
     if (t + kStages - 1 < ntiles) issue(t + kStages - 1);
     cp_async_commit();
-    cp_async_wait<kStages - 1>();
-    __syncthreads();
     T(*tile)[tile_ld<T>()] = tiles[t % kStages];
     if (t < nlead) {  // an earlier off-diagonal block: b -= L_ij x_j
       const int ok = fill_sx(col_block(t));
@@ -568,7 +506,8 @@ fast_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32_
         cp_async_wait<0>();  // no copy may land after the CTA has left
         return;
       }
-      prefetch(t + 1 < nlead ? col_block(t + 1) : pcb);
+      if (t + 1 < nlead) prefetch(col_block(t + 1));
+      else if (kCouple) prefetch(pcb);
       half_product(tile, a, T(-1));
       continue;
     }
@@ -620,7 +559,7 @@ fast_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32_
       if (q < nrhs) {
         const T v = SweepBits<T>::canon(d[q]);
         if (FWD) Y[(r0 + r) + q * ldy] = v;
-        else Out[(r0 + r) + q * ldo] = v;
+        else Out[(TRANS ? (int64_t)perm[r0 + r] : r0 + r) + q * ldo] = v;
       }
 }
 
@@ -746,83 +685,71 @@ void getrs_carve(GetrsPlan<T>& p, void* base, size_t bytes, int64_t work_cols) {
 }
 
 namespace {
-template <typename T, int NR, bool FAST>
-cudaError_t run_chunk(const GetrsPlan<T>& p, char trans, int nr, T* B, int64_t ldb,
-                      cudaStream_t s) {
+template <typename T, int NR, bool TRANS, bool FWD>
+void launch_sweep(const GetrsPlan<T>& p, int nr, T* B, int64_t ldb, cudaStream_t s) {
   const int64_t nblk = (p.n + kTS - 1) / kTS;
-  int32_t* ffwd = p.flags;
-  int32_t* fbwd = p.flags + nblk;
+  const T* In = FWD ? B : nullptr;
+  T* Out = FWD ? nullptr : B;
+  // algorithmic work of one sweep: the triangle (n^2/2 elements) read once,
+  // n^2 flops per right-hand side
+  LaunchScope ls(K_SOLVE, (double)p.n * (double)p.n * nr,
+                 0.5 * (double)p.n * (double)p.n * sizeof(T) + 2.0 * p.n * nr * sizeof(T), s);
+  if (p.fast && p.inv)
+    fast_sweep_kernel<T, NR, TRANS, FWD><<<(unsigned)(nblk * ((nr + NR - 1) / NR)), kSweepThreads, sweep_smem<T>(), s>>>(
+        p.n, p.LU, p.lda, p.perm, In, ldb, p.work, p.n, Out, ldb, nr, p.scratch, p.inv);
+  else
+    solve_sweep_kernel<T, TRANS, FWD><<<(unsigned)(nblk * nr), kSweepThreads, sweep_smem<T>(), s>>>(
+        p.n, p.LU, p.lda, p.perm, In, ldb, p.work, p.n, Out, ldb, nr, p.scratch);
+}
+
+template <typename T, int NR>
+cudaError_t run_chunk(const GetrsPlan<T>& p, char trans, int nr, T* B, int64_t ldb, cudaStream_t s) {
+  const bool tr = trans == 'T' || trans == 't' || trans == 'C' || trans == 'c';
   // dependents poll Y (forward) and B (backward): fill both with the sentinel
   cudaError_t e = cudaMemsetAsync(p.work, 0xFF, (size_t)p.n * nr * sizeof(T), s);
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(&p.scratch->ticket, 0, sizeof(unsigned), s);
   if (e != cudaSuccess) return e;
-  const bool tr = trans == 'T' || trans == 't' || trans == 'C' || trans == 'c';
-  // algorithmic work of one sweep: the triangle (n^2/2 elements) read once,
-  // n^2 flops per right-hand side
-  const double tri_bytes = 0.5 * (double)p.n * (double)p.n * sizeof(T) + 2.0 * p.n * nr * sizeof(T);
-  const double sweep_flops = (double)p.n * (double)p.n * nr;
-  const size_t smem = sweep_smem<T>();
-  {
-    LaunchScope ls(K_SOLVE, sweep_flops, tri_bytes, s);
-    if (FAST && !tr)
-      fast_sweep_kernel<T, NR, true><<<(unsigned)nblk, kSweepThreads, smem, s>>>(
-          p.n, p.LU, p.lda, p.perm, B, ldb, p.work, p.n, nullptr, 0, nr, p.scratch, p.inv);
-    else if (!tr)
-      solve_sweep_kernel<T, NR, false, true, FAST><<<(unsigned)nblk, kSweepThreads, smem, s>>>(
-          p.n, p.LU, p.lda, p.perm, B, ldb, p.work, p.n, nullptr, 0, nr, ffwd, p.scratch, p.inv);
-    else
-      solve_sweep_kernel<T, NR, true, true, FAST><<<(unsigned)nblk, kSweepThreads, smem, s>>>(
-          p.n, p.LU, p.lda, p.perm, B, ldb, p.work, p.n, nullptr, 0, nr, ffwd, p.scratch, p.inv);
-  }
+  if (tr) launch_sweep<T, NR, true, true>(p, nr, B, ldb, s);
+  else launch_sweep<T, NR, false, true>(p, nr, B, ldb, s);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(&p.scratch->ticket, 0, sizeof(unsigned), s);
   if (e != cudaSuccess) return e;
   e = cudaMemset2DAsync(B, ldb * sizeof(T), 0xFF, p.n * sizeof(T), nr, s);
   if (e != cudaSuccess) return e;
-  LaunchScope ls(K_SOLVE, sweep_flops, tri_bytes, s);
-  if (FAST && !tr)
-    fast_sweep_kernel<T, NR, false><<<(unsigned)nblk, kSweepThreads, smem, s>>>(
-        p.n, p.LU, p.lda, p.perm, nullptr, 0, p.work, p.n, B, ldb, nr, p.scratch, p.inv);
-  else if (!tr)
-    solve_sweep_kernel<T, NR, false, false, FAST><<<(unsigned)nblk, kSweepThreads, smem, s>>>(
-        p.n, p.LU, p.lda, p.perm, nullptr, 0, p.work, p.n, B, ldb, nr, fbwd, p.scratch, p.inv);
-  else
-    solve_sweep_kernel<T, NR, true, false, FAST><<<(unsigned)nblk, kSweepThreads, smem, s>>>(
-        p.n, p.LU, p.lda, p.perm, nullptr, 0, p.work, p.n, B, ldb, nr, fbwd, p.scratch, p.inv);
+  if (tr) launch_sweep<T, NR, true, false>(p, nr, B, ldb, s);
+  else launch_sweep<T, NR, false, false>(p, nr, B, ldb, s);
   return cudaGetLastError();
 }
 
 template <typename T, int NR>
-cudaError_t run_chunk_mode(const GetrsPlan<T>& p, char trans, int nr, T* B, int64_t ldb, cudaStream_t s) {
-  return (p.fast && p.inv) ? run_chunk<T, NR, true>(p, trans, nr, B, ldb, s)
-                           : run_chunk<T, NR, false>(p, trans, nr, B, ldb, s);
+void configure_fast() {
+  const int b = (int)sweep_smem<T>();
+  cudaFuncSetAttribute(fast_sweep_kernel<T, NR, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+  cudaFuncSetAttribute(fast_sweep_kernel<T, NR, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+  cudaFuncSetAttribute(fast_sweep_kernel<T, NR, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+  cudaFuncSetAttribute(fast_sweep_kernel<T, NR, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+}
+
+template <typename T>
+void configure_exact() {
+  const int b = (int)sweep_smem<T>();
+  cudaFuncSetAttribute(solve_sweep_kernel<T, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+  cudaFuncSetAttribute(solve_sweep_kernel<T, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+  cudaFuncSetAttribute(solve_sweep_kernel<T, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+  cudaFuncSetAttribute(solve_sweep_kernel<T, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
 }
 }  // namespace
 
-template <typename T, int NR, bool FAST>
-void configure_nr_mode() {
-  const int b = (int)sweep_smem<T>();
-  cudaFuncSetAttribute(solve_sweep_kernel<T, NR, false, true, FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-  cudaFuncSetAttribute(solve_sweep_kernel<T, NR, true, true, FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-  cudaFuncSetAttribute(solve_sweep_kernel<T, NR, false, false, FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-  cudaFuncSetAttribute(solve_sweep_kernel<T, NR, true, false, FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-  if (FAST) {
-    cudaFuncSetAttribute(fast_sweep_kernel<T, NR, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    cudaFuncSetAttribute(fast_sweep_kernel<T, NR, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-  }
-}
-
-template <typename T, int NR>
-void configure_nr() {
-  configure_nr_mode<T, NR, false>();
-  configure_nr_mode<T, NR, true>();
-}
-
 void getrs_configure(int /*device*/) {
-  configure_nr<double, 1>(); configure_nr<double, 2>(); configure_nr<double, 4>(); configure_nr<double, 8>();
-  configure_nr<float, 1>(); configure_nr<float, 2>(); configure_nr<float, 4>(); configure_nr<float, 8>();
+  configure_exact<double>();
+  configure_exact<float>();
+  configure_fast<double, 1>();
+  configure_fast<float, 1>();
+  configure_fast<float, 2>();
+  configure_fast<float, 4>();
+  configure_fast<float, 8>();
 }
 
 template <typename T>
@@ -834,10 +761,12 @@ cudaError_t getrs_launch(const GetrsPlan<T>& p, char trans, int64_t nrhs, T* B, 
     int nr = (int)std::min<int64_t>(chunk, nrhs - c);
     T* Bc = B + c * ldb;
     cudaError_t e;
-    if (nr == 1) e = run_chunk_mode<T, 1>(p, trans, nr, Bc, ldb, s);
-    else if (nr == 2) e = run_chunk_mode<T, 2>(p, trans, nr, Bc, ldb, s);
-    else if (nr <= 4) e = run_chunk_mode<T, 4>(p, trans, nr, Bc, ldb, s);
-    else e = run_chunk_mode<T, 8>(p, trans, nr, Bc, ldb, s);
+    if (sizeof(T) == 8 || nr == 1) e = run_chunk<T, 1>(p, trans, nr, Bc, ldb, s);
+    else if constexpr (sizeof(T) == 4) {
+      if (nr == 2) e = run_chunk<T, 2>(p, trans, nr, Bc, ldb, s);
+      else if (nr <= 4) e = run_chunk<T, 4>(p, trans, nr, Bc, ldb, s);
+      else e = run_chunk<T, 8>(p, trans, nr, Bc, ldb, s);
+    }
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;

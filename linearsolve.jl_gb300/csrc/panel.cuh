@@ -27,27 +27,14 @@ __device__ __forceinline__ T key_magnitude(typename PivKey<T>::K key) {
 // arithmetic without a branch.  The library division is a chain of dependent
 // FP64 instructions (about 70 cycles each here, 600 in place) behind a branch
 // the scheduler cannot move a warp reduction across; this takes about 230 and
-// interleaves.  The significand's reciprocal comes from Newton's iteration on
-// fixed-point words started from the hardware approximation (22 bits -> 43 ->
-// 60); the quotient's last unit and its rounding are settled by the exact
-// remainder modulo 2^64 (it is smaller than four divisors).  A tie cannot
-// occur: 2^k = m (2 q + 1) only for m = 1.
+// interleaves.  The quotient's last unit and its rounding are settled by the
+// exact remainder modulo 2^64 (it is smaller than four divisors).  A tie
+// cannot occur: 2^k = m (2 q + 1) only for m = 1.
 __device__ __forceinline__ double recip_normal(double x) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | (1ull << 52);
   const int e = (int)(b >> 52);
-  const unsigned long long d = m << 11;             // 2^63 <= d < 2^64
-  const unsigned dh = (unsigned)(d >> 32), dl = (unsigned)d;
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint2float_rz(dh)));
-  // r0 ~ 2^63 / dh, below 2^32
-  const unsigned r0 = (unsigned)min((unsigned long long)__float2ull_rz(y * 9.2233720368547758e18f), 0xFFFFFFFFull);
-  // 2^63 - r0 d / 2^32, about 41 bits, and the first step: R1 ~ 2^127 / d
-  const long long e1 = (long long)((1ull << 63) - ((unsigned long long)r0 * dh + __umulhi(r0, dl)));
-  const unsigned long long R1 = ((unsigned long long)r0 << 32) + (unsigned long long)(((long long)(int)(e1 >> 12) * (long long)(r0 >> 1)) >> 18);
-  const long long e2 = (long long)((1ull << 63) - __umul64hi(R1, d));
-  const unsigned long long R2 = R1 + (unsigned long long)(((long long)(int)(e2 >> 1) * (long long)(R1 >> 33)) >> 29);
-  unsigned long long q = R2 >> 11;                  // ~ 2^105 / m
+  unsigned long long q = recip_word(m) >> 11;       // ~ 2^105 / m
   long long rem = -(long long)(q * m);              // 2^105 - q m
   const long long ms = (long long)m;
 #pragma unroll

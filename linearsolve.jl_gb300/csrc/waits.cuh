@@ -27,6 +27,7 @@ struct SweepBits<double> {
     return v;
   }
   static __device__ __forceinline__ double as_t(U v) { return __longlong_as_double((long long)v); }
+  static __device__ __forceinline__ U bits(double v) { return (U)__double_as_longlong(v); }
   // NaN -> the canonical quiet NaN, on the integer pipe
   static __device__ __forceinline__ double canon(double v) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(v);
@@ -43,6 +44,7 @@ struct SweepBits<float> {
     return v;
   }
   static __device__ __forceinline__ float as_t(U v) { return __uint_as_float(v); }
+  static __device__ __forceinline__ U bits(float v) { return __float_as_uint(v); }
   static __device__ __forceinline__ float canon(float v) {
     return (__float_as_uint(v) << 1) > 0xff000000u ? __uint_as_float(0x7fc00000u) : v;
   }
