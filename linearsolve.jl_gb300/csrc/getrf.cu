@@ -484,83 +484,96 @@ laswp_moves_kernel(T* __restrict__ A, int64_t lda, int64_t ncols_total, int64_t 
 // Unit-lower TRSM base case: B[0:k, cols] := L \ B with L = k x k (k <= KM,
 // KM = 64 or 128) held in shared memory.  One warp per right-hand-side
 // column: lane l holds rows l, l + 32, ... in registers; x_kk is broadcast
-// with a shuffle and every row below it is updated, kk ascending
-// (blocked_lufact.jl:146-178 order).  Row blocks of 32 that are already
-// final are skipped with a warp-uniform branch, so finished rows cost no
-// (FP64) instructions.
+// with a shuffle and every row block from kk's on is updated, kk ascending
+// (blocked_lufact.jl:146-178 order).  Nothing is masked: a row's value is
+// kept aside when it is final (`own`), what its register goes through after
+// that, and rows past k, are not used.
+//
+// Bound: FP64, the FP64 pipe for many columns (k = 128: 320 instructions a
+// column, 16.5 cycles each on an SM) and the chain (a shuffle and an FP64
+// instruction a step, 108 cycles) for few; FP32, the chain and the issue of 16
+// warps.  All of a factorization's TRSM launches (events, ~5 us each of it
+// launch), against one masked step at a time and 8-byte copies by as few as one
+// warp: FP64 n = 1000 0.67 -> 0.40 ms, n = 8192 14.2 -> 9.2 ms, FP32 n = 3001
+// 1.26 -> 0.87 ms.
 constexpr int kTrsmMax = 128;
-// warps per CTA: one CTA holds the L block; the FP32 128-row variant runs
-// more columns per CTA, while FP64 keeps more CTAs (each SM's FP64 pipe is
-// the limit, so the columns should spread over as many SMs as possible)
-template <typename T, int KM>
-__host__ __device__ constexpr int trsm_warps() { return (sizeof(T) == 4 && KM == 128) ? 16 : 8; }
+template <typename T>
+__host__ __device__ constexpr int trsm_warps_max() { return sizeof(T) == 4 ? 16 : 8; }
 
 template <typename T, int KM>
-__global__ void __launch_bounds__(trsm_warps<T, KM>() * 32)
+__global__ void __launch_bounds__(trsm_warps_max<T>() * 32)
 trsm_lunit_kernel(const T* __restrict__ L, int64_t ldl, int k, T* __restrict__ B,
                   int64_t ldb, int64_t ncols) {
   constexpr int RPL = KM / 32;  // rows per lane
-  // warps (columns in flight) of this CTA: chosen per launch for FP64, fixed
-  // for FP32 (a compile-time stride keeps its short chain steps lean)
-  const int nw = sizeof(T) == 8 ? (int)(blockDim.x >> 5) : trsm_warps<T, KM>();
+  constexpr int V = 16 / (int)sizeof(T);
+  const int nw = (int)(blockDim.x >> 5);
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T(*sL)[KM + 1] = reinterpret_cast<T(*)[KM + 1]>(smem_raw);  // sL[c][r] = L[r, c]
+  T(*sL)[KM] = reinterpret_cast<T(*)[KM]>(smem_raw);  // sL[c][r] = L[r, c], r > c
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if constexpr (sizeof(T) == 8) {
-    // the strictly lower triangle of L, copied asynchronously (an FP64 CTA
-    // may have a single warp)
-    for (int c = warp; c < k; c += nw)
-      for (int r = c + 1 + lane; r < k; r += 32) {
+  const int64_t stride = (int64_t)gridDim.x * nw;
+  int64_t col = (int64_t)blockIdx.x * nw + warp;
+  T v[RPL];
+  auto load = [&](int64_t c) {
+#pragma unroll
+    for (int q = 0; q < RPL; ++q) v[q] = lane + 32 * q < k ? B[lane + 32 * q + c * ldb] : T(0);
+  };
+  // the columns below the diagonal, all copies in flight at once; in 16-byte
+  // words where the block is aligned and no word reaches past row k - 1
+  const bool vec = ((reinterpret_cast<uintptr_t>(L) | (uintptr_t)(ldl * (int64_t)sizeof(T))) & 15) == 0 && k % V == 0;
+  if (vec) {
+    constexpr int CPC = KM / V;  // words per column
+    for (int idx = threadIdx.x; idx < k * CPC; idx += blockDim.x) {
+      const int c = idx / CPC, r = (idx % CPC) * V;
+      if (r + V > c + 1 && r < k) {
         const unsigned d = (unsigned)__cvta_generic_to_shared(&sL[c][r]);
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(L + r + (int64_t)c * ldl)
-                     : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(L + r + (int64_t)c * ldl) : "memory");
       }
-    asm volatile("cp.async.wait_all;" ::: "memory");
+    }
   } else {
-    // asynchronous copies, all in flight at once (a load-store loop waits
-    // out one global latency per element); a fixed thread count keeps the
-    // index arithmetic compile-time
-    constexpr int NT = trsm_warps<T, KM>() * 32;
-#pragma unroll
-    for (int e = 0; e < KM * KM / NT; ++e) {
-      const int idx = e * NT + (int)threadIdx.x, c = idx / KM, r = idx % KM;
-      if (c < k && r > c && r < k) {
+    for (int idx = threadIdx.x; idx < k * KM; idx += blockDim.x) {
+      const int c = idx / KM, r = idx % KM;
+      if (r > c && r < k) {
         const unsigned d = (unsigned)__cvta_generic_to_shared(&sL[c][r]);
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(L + r + (int64_t)c * ldl)
-                     : "memory");
+        if constexpr (sizeof(T) == 8)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(L + r + (int64_t)c * ldl) : "memory");
+        else
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(L + r + (int64_t)c * ldl) : "memory");
       }
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
   }
+  if (col < ncols) load(col);
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
-  for (int64_t col = (int64_t)blockIdx.x * nw + warp; col < ncols; col += (int64_t)gridDim.x * nw) {
-    T* b = B + col * ldb;
-    T v[RPL];
+  for (; col < ncols; col += stride) {
 #pragma unroll
-    for (int q = 0; q < RPL; ++q) v[q] = lane + 32 * q < k ? b[lane + 32 * q] : T(0);
-    for (int kk = 0; kk < k - 1; ++kk) {
-      const int qk = kk >> 5;
-      T src = v[0];
+    for (int b = 0; b < RPL; ++b) {
+      if (32 * b >= k) break;
+      T own = T(0);
+      const int kend = min(32, k - 32 * b);
+#pragma unroll 8
+      for (int i = 0; i < 32; ++i) {
+        if (i >= kend) break;
+        const T x = __shfl_sync(0xffffffffu, v[b], i);
+        own = lane == i ? x : own;
+        const T* l = sL[32 * b + i] + lane;
 #pragma unroll
-      for (int q = 1; q < RPL; ++q)
-        if (qk == q) src = v[q];
-      const T xk = __shfl_sync(0xffffffffu, src, kk & 31);
-#pragma unroll
-      for (int q = 0; q < RPL; ++q) {
-        if (q < qk) continue;  // rows 32q..32q+31 are final
-        if (sizeof(T) == 8 && 32 * q >= k) break;  // no rows (a predicated-off FP64 FMA still occupies the pipe)
-        const int r = lane + 32 * q;
-        if (r > kk && r < k) v[q] = fma(-sL[kk][r], xk, v[q]);
+        for (int q = b; q < RPL; ++q) {
+          if (q > b && 32 * q >= k) break;
+          v[q] = fma(-l[32 * q], x, v[q]);
+        }
       }
+      v[b] = own;
     }
+    T* bc = B + col * ldb;
 #pragma unroll
     for (int q = 0; q < RPL; ++q)
-      if (lane + 32 * q < k) b[lane + 32 * q] = v[q];
+      if (lane + 32 * q < k) bc[lane + 32 * q] = v[q];
+    if (col + stride < ncols) load(col + stride);
   }
 }
 
 template <typename T, int KM>
-constexpr size_t trsm_smem() { return (size_t)KM * (KM + 1) * sizeof(T); }
+constexpr size_t trsm_smem() { return (size_t)KM * KM * sizeof(T); }
 
 // ---------------------------------------------------------------------------
 // TRSM base blocks of the 16-bit-operand factors (FP32 working matrix; the
@@ -1196,14 +1209,12 @@ struct Driver {
     }
     if (k <= p.trsm_base && k <= kTrsmMax) {
       const DeviceInfo& di = device_info(device);
-      // one column per warp.  FP64: few columns are spread over the SMs one
-      // or two warps per CTA (each column is a chain of k dependent steps of
-      // 64-cycle FMAs, and the warps of one SM share its FP64 pipe); FP32
-      // chains are short and keep full CTAs.
-      const int maxw = k <= 64 ? trsm_warps<T, 64>() : trsm_warps<T, 128>();
-      const int warps = sizeof(T) == 4 ? maxw
-                                       : (int)std::max<int64_t>(1, std::min<int64_t>(maxw, (ncols + di.num_sms - 1) / di.num_sms));
-      unsigned blocks = (unsigned)std::min<int64_t>((ncols + warps - 1) / warps, (int64_t)di.num_sms * 8);
+      // One column per warp.  FP64: four warps saturate an SM's FP64 pipe while
+      // they all issue; eight when the columns fill the SMs more than once
+      // (their chains then overlap).  FP32: 16 where there are columns enough.
+      const int64_t per_sm = (ncols + di.num_sms - 1) / di.num_sms;
+      const int warps = sizeof(T) == 4 ? (per_sm > 8 ? 16 : 8) : (per_sm > 4 ? 8 : 4);
+      unsigned blocks = (unsigned)std::min<int64_t>((ncols + warps - 1) / warps, (int64_t)di.num_sms * (k <= 64 ? 4 : 1));
       LaunchScope ls(K_TRSM, (double)k * (k - 1) * ncols, (2.0 * k * ncols + (double)k * k) * sizeof(T), s);
       if (k <= 64)
         trsm_lunit_kernel<T, 64><<<blocks, warps * 32, trsm_smem<T, 64>(), s>>>(
@@ -1283,6 +1294,8 @@ void getrf_configure(int device) {
                        (int)trsm_smem<double, 128>());
   cudaFuncSetAttribute(trsm_lunit_kernel<float, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)trsm_smem<float, 128>());
+  cudaFuncSetAttribute(trsm_lunit_kernel<double, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)trsm_smem<double, 64>());
   cudaFuncSetAttribute(perm_from_ipiv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (kPermSmemMax + kPermChunk) * (int)sizeof(int32_t));
   getrs_configure(device);

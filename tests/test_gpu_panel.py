@@ -84,3 +84,12 @@ def test_integer_reciprocal_matches_ieee():
     m64, m32 = ctypes.c_uint64(), ctypes.c_uint64()
     assert lib.gblu_tool_recipcheck(1 << 24, 99, ctypes.byref(m64), ctypes.byref(m32)) == 0
     assert m64.value == 0 and m32.value == 0, (m64.value, m32.value)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("m", [1, 31, 33, 63, 64, 65, 95, 127, 128, 130])
+@pytest.mark.parametrize("extra", [1, 3, 700])
+def test_wide_trsm_bit_exact(pkg, oracle_mod, dtype, m, extra):
+    """U12 := L11 \\ A12 of a wide matrix: orders around the 32-row blocks, the
+    16-byte and the element copies of L, few and many columns."""
+    _check(pkg, oracle_mod, np.random.default_rng(m + extra).standard_normal((m, m + extra)).astype(dtype))
