@@ -376,42 +376,63 @@ __global__ void colmax_kernel(int64_t n, int W, const double* __restrict__ X, in
   }
 }
 
-// Per-column power-of-two scale from the column maxima (bit patterns):
-// sc[q] = 1 / 2^ilogb(max), sc[kMaxW + q] = 2^ilogb(max) (1 for a zero or
-// non-finite maximum), so the FP32 right-hand side is O(1).
-__global__ void pow2_scales_kernel(int W, const unsigned long long* __restrict__ colmax,
-                                   double* __restrict__ sc) {
-  const int q = threadIdx.x;
-  if (q >= W) return;
-  const double m = __longlong_as_double((long long)colmax[q]);
-  const double scale = (m > 0 && isfinite(m)) ? ldexp(1.0, ilogb(m)) : 1.0;
-  sc[q] = 1.0 / scale;
-  sc[kMaxW + q] = scale;
-}
-
-// D[:,q] = float(R[:,q] * inv_scale[q])
-__global__ void scale_to_f32_kernel(int64_t n, int W, const double* __restrict__ R, int64_t ldr,
-                                    const double* __restrict__ inv_scale, float* __restrict__ D,
-                                    int64_t ldd) {
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < n * W;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    int q = (int)(idx / n);
-    int64_t i = idx - (int64_t)q * n;
-    D[i + q * ldd] = (float)(R[i + q * ldr] * inv_scale[q]);
+// The power-of-two scale 2^ilogb(m) of a column from its maximum's bit pattern
+// (1 for a zero or non-finite maximum), and its inverse, so the FP32
+// right-hand side is O(1).
+__device__ __forceinline__ void pow2_scale(unsigned long long bits, double& scale, double& inv) {
+  const unsigned long long e = bits >> 52;  // m >= 0
+  if (e - 1ull < 2045ull) {
+    scale = __longlong_as_double((long long)(e << 52));
+    inv = __longlong_as_double((long long)((2046ull - e) << 52));
+    return;
   }
+  const double m = __longlong_as_double((long long)bits);
+  scale = (m > 0 && isfinite(m)) ? ldexp(1.0, ilogb(m)) : 1.0;
+  inv = 1.0 / scale;
 }
 
-// X[:,q] = beta*X[:,q] + scale[q] * double(D[:,q])
+// D[:,q] = float(R[:,q] / scale_q), scale_q from the column maximum colmax[q]
+__global__ void scale_to_f32_kernel(int64_t n, int W, const double* __restrict__ R, int64_t ldr,
+                                    const unsigned long long* __restrict__ colmax, float* __restrict__ D,
+                                    int64_t ldd) {
+  const int q = blockIdx.y;
+  double scale, inv;
+  pow2_scale(colmax[q], scale, inv);
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    D[i + q * ldd] = (float)(R[i + q * ldr] * inv);
+}
+
+// X[:,q] = scale_q * double(D[:,q])
 __global__ void update_from_f32_kernel(int64_t n, int W, double* __restrict__ X, int64_t ldx,
                                        const float* __restrict__ D, int64_t ldd,
-                                       const double* __restrict__ scale, double beta) {
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < n * W;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    int q = (int)(idx / n);
-    int64_t i = idx - (int64_t)q * n;
-    double d = scale[q] * (double)D[i + q * ldd];
-    X[i + q * ldx] = beta == 0.0 ? d : fma(beta, X[i + q * ldx], d);
+                                       const unsigned long long* __restrict__ colmax) {
+  const int q = blockIdx.y;
+  double scale, inv;
+  pow2_scale(colmax[q], scale, inv);
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    X[i + q * ldx] = scale * (double)D[i + q * ldd];
+}
+
+// The correction of refinement: X[:,q] += scale_q * double(D[:,q]) for the
+// columns of `active`, and max |X[:,q]| of every column into xmax.
+__global__ void __launch_bounds__(256)
+correct_kernel(int64_t n, unsigned active, double* __restrict__ X, int64_t ldx, const float* __restrict__ D,
+               int64_t ldd, const unsigned long long* __restrict__ colmax, unsigned long long* __restrict__ xmax) {
+  const int q = blockIdx.y;
+  double scale, inv;
+  pow2_scale(colmax[q], scale, inv);
+  const bool on = (active >> q) & 1u;
+  double mx = 0.0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    double x = X[i + q * ldx];
+    if (on) {
+      x += scale * (double)D[i + q * ldd];
+      X[i + q * ldx] = x;
+    }
+    const double av = fabs(x);
+    mx = (av > mx || isnan(av)) ? av : mx;
   }
+  block_max_into(mx, xmax + q);
 }
 
 // Sum of squares of each of W columns, in two fixed-order passes: block b of
@@ -453,15 +474,105 @@ __global__ void sumsq_final_kernel(int W, const double* __restrict__ part, doubl
 // gflags[2q + 1] = basis size k.  A column that stopped keeps its state and
 // gets 1/norm = 0, so its later basis vectors are zero and stay finite.
 
-// beta_q = ||z_q||_2 from the squared norm in hn2[q] (columns outside run_mask
-// do not step), g = beta e_1.
-__global__ void gmres_begin_kernel(int nc, unsigned run_mask, const double* __restrict__ hn2,
+// Classical Gram-Schmidt, twice, of z_q = V_q(:, j + 1) against V_q(:, 0 .. j)
+// for every column q of a block at once, kGsRows rows a CTA, in three launches.
+// At ordinary sizes the step is bound by the latency of its launches, not by
+// bytes (n = 3000, four columns: 96 KB a basis vector): two GEMV pairs and a
+// norm per column, forty launches a step, took the solve 21.9 ms; these three
+// with the scaling folded into the conversions, 15.9 ms.  256 rows a CTA keep
+// the partial sums the next launch adds short (12 at n = 3000, 64 at 16384).
+// Every launch leaves partial sums per CTA; the next one adds them in CTA
+// order, so a column's result does not depend on the others.
+//   mode 0: partials of V^T z
+//   mode 1: h = sum of `in`; z -= V h; partials of V^T z
+//   mode 2: h = sum of `in`; z -= V h; partials of z . z
+//   mode 3: partials of z . z
+// in / out: [q][i][CTA], i <= j (dots) or one (norm); h + q * hq: h_0 .. h_j.
+constexpr int kGsRows = 256;
+__global__ void __launch_bounds__(kGsRows)
+gmres_gs_kernel(int mode, int64_t n, int j, double* __restrict__ V, int64_t ldV, const double* __restrict__ in,
+                double* __restrict__ out, double* __restrict__ h, int64_t hq) {
+  __shared__ double zs[kGsRows];
+  __shared__ double hs[kGmresRestart + 1];
+  const int q = blockIdx.y, blk = blockIdx.x, nblk = gridDim.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t r0 = (int64_t)blk * kGsRows, row = r0 + tid;
+  double* Vq = V + (size_t)q * ldV;
+  double* z = Vq + (size_t)(j + 1) * n;
+  double zr = row < n ? z[row] : 0.0;
+  if (mode == 1 || mode == 2) {
+    if (tid <= j) {
+      const double* p = in + ((size_t)q * (kGmresRestart + 1) + tid) * nblk;
+      double sum = 0.0;
+#pragma unroll 8
+      for (int b = 0; b < nblk; ++b) sum += p[b];
+      hs[tid] = sum;
+      if (blk == 0) h[(size_t)q * hq + tid] = sum;
+    }
+    __syncthreads();
+    if (row < n) {
+#pragma unroll 4
+      for (int i = 0; i <= j; ++i) zr = fma(-Vq[(size_t)i * n + row], hs[i], zr);
+      z[row] = zr;
+    }
+  }
+  zs[tid] = zr;
+  __syncthreads();
+  if (mode <= 1) {
+    for (int i = warp; i <= j; i += kGsRows / 32) {
+      const double* v = Vq + (size_t)i * n + r0;
+      double acc = 0.0;
+#pragma unroll
+      for (int k = 0; k < kGsRows / 32; ++k) {
+        const int r = lane + 32 * k;
+        const double x = r0 + r < n ? v[r] : 0.0;
+        acc = fma(x, zs[r], acc);
+      }
+      for (int off = 16; off; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
+      if (lane == 0) out[((size_t)q * (kGmresRestart + 1) + i) * nblk + blk] = acc;
+    }
+  } else if (warp == 0) {
+    double acc = 0.0;
+#pragma unroll
+    for (int k = 0; k < kGsRows / 32; ++k) acc = fma(zs[lane + 32 * k], zs[lane + 32 * k], acc);
+    for (int off = 16; off; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
+    if (lane == 0) out[(size_t)q * nblk + blk] = acc;
+  }
+}
+
+// X[:,q] += V_q(:, 0 .. k_q - 1) y_q for the basis sizes k_q in gflags.
+__global__ void __launch_bounds__(256)
+gmres_combine_kernel(int64_t n, const double* __restrict__ V, int64_t ldV, const double* __restrict__ y,
+                     const int* __restrict__ gflags, double* __restrict__ X, int64_t ldx) {
+  const int q = blockIdx.y;
+  const int k = gflags[2 * q + 1];
+  if (k == 0) return;
+  const double* Vq = V + (size_t)q * ldV;
+  const double* yq = y + (size_t)q * (kGmresRestart + 1);
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    double acc = 0.0;
+#pragma unroll 4
+    for (int c = 0; c < k; ++c) acc = fma(Vq[(size_t)c * n + i], yq[c], acc);
+    X[i + q * ldx] += acc;
+  }
+}
+
+// ||z_q||_2 from the CTAs' partial sums of squares.
+__device__ __forceinline__ double norm_of(const double* __restrict__ pn, int q, int nblk) {
+  double sum = 0.0;
+#pragma unroll 8
+  for (int b = 0; b < nblk; ++b) sum += pn[(size_t)q * nblk + b];
+  return sqrt(sum);
+}
+
+// beta_q = ||z_q||_2 (columns outside run_mask do not step), g = beta e_1.
+__global__ void gmres_begin_kernel(int nc, unsigned run_mask, const double* __restrict__ pn, int nblk,
                                    double* __restrict__ gm, int* __restrict__ gflags) {
   const int q = threadIdx.x;
   if (q >= nc) return;
   double* st = gm + (size_t)q * kGmStride;
   int* fl = gflags + 2 * q;
-  const double beta = ((run_mask >> q) & 1u) ? sqrt(hn2[q]) : 0.0;
+  const double beta = ((run_mask >> q) & 1u) ? norm_of(pn, q, nblk) : 0.0;
   const bool step = beta > 0 && isfinite(beta);
   for (int i = 0; i <= kGmresRestart; ++i) {
     st[kGmG + i] = 0.0;
@@ -487,10 +598,11 @@ __global__ void gmres_scale_kernel(int64_t n, int nc, double* __restrict__ V, in
 }
 
 // Step j of each stepping column: Hessenberg column from the two projection
-// passes and the norm (h: [q][pass 0, 1, norm^2][m + 1]), the previous Givens
+// passes (h: [q][pass 0, 1, -][m + 1]) and the norm's partials, the previous Givens
 // rotations, the new rotation, g, the stopping test |g_{j+1}| <= rtol beta.
-__global__ void gmres_step_kernel(int nc, int j, int m, const double* __restrict__ h, double rtol,
-                                  double* __restrict__ gm, int* __restrict__ gflags) {
+__global__ void gmres_step_kernel(int nc, int j, int m, const double* __restrict__ h,
+                                  const double* __restrict__ pn, int nblk, double rtol, double* __restrict__ gm,
+                                  int* __restrict__ gflags) {
   const int q = threadIdx.x;
   if (q >= nc) return;
   double* st = gm + (size_t)q * kGmStride;
@@ -502,7 +614,7 @@ __global__ void gmres_step_kernel(int nc, int j, int m, const double* __restrict
   const int hs = kGmresRestart + 1;
   const double* h1 = h + (size_t)(q * 3) * hs;
   const double* h2 = h1 + hs;
-  const double hn = sqrt(h1[2 * hs]);
+  const double hn = norm_of(pn, q, nblk);
   double* Hj = st + kGmH + (size_t)j * (m + 1);
   double* cs = st + kGmCs;
   double* sn = st + kGmSn;
@@ -549,14 +661,6 @@ __global__ void gmres_finish_kernel(int nc, int m, const double* __restrict__ gm
     const double d = H[(size_t)i * (m + 1) + i];
     y[i] = d != 0 ? acc / d : 0.0;
   }
-}
-
-// Y = a*X + b*Y
-__global__ void axpby_kernel(int64_t n, double a, const double* __restrict__ X, double b,
-                             double* __restrict__ Y) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    Y[i] = b == 0.0 ? a * X[i] : fma(a, X[i], b * Y[i]);
 }
 
 // ---------------------------------------------------------------------------
@@ -784,25 +888,13 @@ struct Solver {
   cudaStream_t s;
   int64_t n;
 
-  // out (len n, W cols) <- M^{-1} v using the FP32 factors with a per-column
-  // power-of-two scale so the FP32 right-hand side is O(1).  No host sync.
-  int32_t precond(const double* v, int64_t ldv, double* out, int64_t ldo, int W) {
-    unsigned long long* cm = w.colmax + 3 * w.W;
-    double* dsc = w.anorm_dev;  // 2*kMaxW doubles of scale storage
-    GBLU_CK(ctx, cudaMemsetAsync(cm, 0, W * sizeof(unsigned long long), s), "memset");
+  // w.d32 (W cols) <- LU^{-1} (v / scale), with the FP32 factors and each
+  // column's power-of-two scale (from its maximum, cm), so the FP32
+  // right-hand side is O(1).  No host sync.
+  int32_t precond_f32(const double* v, int64_t ldv, int W, const unsigned long long* cm) {
     {
       LaunchScope ls_(K_REFINE, 0.0, 0.0, s);
-      colmax_kernel<<<grid_for(n), 256, 0, s>>>(n, W, v, ldv, cm);
-    }
-    GBLU_CK(ctx, cudaGetLastError(), "colmax");
-    {
-      LaunchScope ls_(K_REFINE, 0.0, 0.0, s);
-      pow2_scales_kernel<<<1, 32, 0, s>>>(W, cm, dsc);
-    }
-    GBLU_CK(ctx, cudaGetLastError(), "scales");
-    {
-      LaunchScope ls_(K_REFINE, 0.0, 0.0, s);
-      scale_to_f32_kernel<<<grid_for(n * W), 256, 0, s>>>(n, W, v, ldv, dsc, w.d32, n);
+      scale_to_f32_kernel<<<dim3(grid_for(n), W), 256, 0, s>>>(n, W, v, ldv, cm, w.d32, n);
     }
     GBLU_CK(ctx, cudaGetLastError(), "scale");
     // RBT factors: d := W1^T d / 2, LU solve, d := W2 d / 2 with (W1, W2) =
@@ -812,22 +904,45 @@ struct Solver {
     if (rbt) GBLU_CK(ctx, rbt_vec_launch(n, W, w.d32, n, f->rbt, side_in, true, s), "butterfly");
     GBLU_CK(ctx, getrs_launch<float>(f->rs32, trans, W, w.d32, n, nullptr, s), "FP32 getrs");
     if (rbt) GBLU_CK(ctx, rbt_vec_launch(n, W, w.d32, n, f->rbt, 1 - side_in, false, s), "butterfly");
+    return GBLU_OK;
+  }
+
+  // out (len n, W cols) <- M^{-1} v
+  int32_t precond(const double* v, int64_t ldv, double* out, int64_t ldo, int W, const unsigned long long* cm) {
+    int32_t st = precond_f32(v, ldv, W, cm);
+    if (st) return st;
     {
       LaunchScope ls_(K_REFINE, 0.0, 0.0, s);
-      update_from_f32_kernel<<<grid_for(n * W), 256, 0, s>>>(n, W, out, ldo, w.d32, n, dsc + kMaxW, 0.0);
+      update_from_f32_kernel<<<dim3(grid_for(n), W), 256, 0, s>>>(n, W, out, ldo, w.d32, n, cm);
     }
     GBLU_CK(ctx, cudaGetLastError(), "update");
     return GBLU_OK;
   }
 
-  // r = b - op(A) x for W columns; returns |r|_inf and |x|_inf per column.
-  int32_t residual(int W, double* rnorm, double* xnorm) {
-    GBLU_CK(ctx, cudaMemsetAsync(w.colmax, 0, 2 * w.W * sizeof(unsigned long long), s), "memset");
+  // x[:,q] += M^{-1} r[:,q] for the columns of `active`; leaves max |x[:,q]|
+  // in w.colmax + w.W (r's maxima are in w.colmax).
+  int32_t correct(int W, unsigned active) {
+    int32_t st = precond_f32(w.r, n, W, w.colmax);
+    if (st) return st;
+    GBLU_CK(ctx, cudaMemsetAsync(w.colmax + w.W, 0, w.W * sizeof(unsigned long long), s), "memset");
+    {
+      LaunchScope ls_(K_REFINE, 0.0, 0.0, s);
+      correct_kernel<<<dim3(grid_for(n), W), 256, 0, s>>>(n, active, w.x, n, w.d32, n, w.colmax, w.colmax + w.W);
+    }
+    GBLU_CK(ctx, cudaGetLastError(), "correction");
+    return GBLU_OK;
+  }
+
+  // r = b - op(A) x for W columns; returns |r|_inf and |x|_inf per column
+  // (x_known: the latter are in w.colmax + w.W already).
+  int32_t residual(int W, double* rnorm, double* xnorm, bool x_known = false) {
+    GBLU_CK(ctx, cudaMemsetAsync(w.colmax, 0, (x_known ? 1 : 2) * w.W * sizeof(unsigned long long), s), "memset");
     GBLU_CK(ctx, gemv(trans == 'N' ? 'N' : 'T', n, n, f->lu64, f->ld, w.x, n, W, -1.0, w.b, n, 1.0,
                       w.r, n, w.partial, w.colmax, s),
             "residual");
-    { LaunchScope ls_(K_REFINE, 0.0, 0.0, s);
-    colmax_kernel<<<grid_for(n), 256, 0, s>>>(n, W, w.x, n, w.colmax + w.W);
+    if (!x_known) {
+      LaunchScope ls_(K_REFINE, 0.0, 0.0, s);
+      colmax_kernel<<<grid_for(n), 256, 0, s>>>(n, W, w.x, n, w.colmax + w.W);
     }
     GBLU_CK(ctx, cudaGetLastError(), "colmax");
     std::vector<unsigned long long> bits(2 * w.W);
@@ -882,18 +997,25 @@ struct Solver {
       GBLU_CK(ctx, cudaMallocHost(&p, 4 * kMaxW * sizeof(int)), "pinned GMRES flags");
       w.gflags_host = reinterpret_cast<int*>(p);
     }
-    int32_t st = precond(w.r, n, V, ldV, nc);
+    const int nblk = (int)((n + kGsRows - 1) / kGsRows);
+    const dim3 gs_grid(nblk, nc);
+    double* p1 = w.partial;  // partial sums of the two projections and of the norm
+    double* p2 = p1 + (size_t)nc * hs * nblk;
+    double* pn = p2 + (size_t)nc * hs * nblk;
+    auto gs = [&](int mode, int j, const double* in, double* out, double* h) {
+      LaunchScope ls_(K_REFINE, (mode == 3 ? 2.0 : 4.0 * (j + 1)) * n * nc, 8.0 * (j + 2) * n * nc, s);
+      gmres_gs_kernel<<<gs_grid, kGsRows, 0, s>>>(mode, n, j, V, ldV, in, out, h, 3 * hs);
+    };
+    unsigned long long* cm = w.colmax + 3 * w.W;  // maxima of the matvec's columns
+    int32_t st = precond(w.r, n, V, ldV, nc, w.colmax);
     if (st) return st;
     unsigned mask = 0;
     for (int q = 0; q < nc; ++q)
-      if (run[q]) {
-        mask |= 1u << q;
-        GBLU_CK(ctx, gemv('T', n, 1, Vq(q, 0), n, Vq(q, 0), n, 1, 1.0, nullptr, 1, 0.0, w.h + q, 1,
-                          w.partial, nullptr, s), "norm");
-      }
+      if (run[q]) mask |= 1u << q;
+    gs(3, -1, nullptr, pn, nullptr);
     {
       LaunchScope ls_(K_REFINE, 0.0, 0.0, s);
-      gmres_begin_kernel<<<1, 32, 0, s>>>(nc, mask, w.h, w.gm, w.gflags);
+      gmres_begin_kernel<<<1, 32, 0, s>>>(nc, mask, pn, nblk, w.gm, w.gflags);
     }
     {
       LaunchScope ls_(K_REFINE, 0.0, 16.0 * n * nc, s);
@@ -909,28 +1031,22 @@ struct Solver {
     int32_t rc = GBLU_OK;
     for (int j = 0; j < m && mask && rc == GBLU_OK; ++j) {
       // w = op(A) v_j ; z = M^{-1} w  (all nc columns at once)
-      cudaError_t ce = gemv(trans == 'N' ? 'N' : 'T', n, n, f->lu64, f->ld, Vq(0, j), ldV, nc, 1.0, nullptr,
-                            1, 0.0, w.w, n, w.partial, nullptr, s);
+      cudaError_t ce = cudaMemsetAsync(cm, 0, nc * sizeof(unsigned long long), s);
+      if (ce == cudaSuccess)
+        ce = gemv(trans == 'N' ? 'N' : 'T', n, n, f->lu64, f->ld, Vq(0, j), ldV, nc, 1.0, nullptr, 1, 0.0, w.w, n,
+                  w.partial, cm, s);
       if (ce != cudaSuccess) { rc = cuda_fail(ctx, ce, "matvec"); break; }
-      rc = precond(w.w, n, Vq(0, j + 1), ldV, nc);
+      rc = precond(w.w, n, Vq(0, j + 1), ldV, nc, cm);
       if (rc) break;
       // classical Gram-Schmidt, twice, and the norm, for every column
-      for (int q = 0; q < nc && ce == cudaSuccess; ++q) {
-        double* z = Vq(q, j + 1);
-        for (int pass = 0; pass < 2 && ce == cudaSuccess; ++pass) {
-          double* hq = w.h + (size_t)(q * 3 + pass) * hs;
-          ce = gemv('T', n, j + 1, Vq(q, 0), n, z, n, 1, 1.0, nullptr, 1, 0.0, hq, 1, w.partial, nullptr, s);
-          if (ce == cudaSuccess)
-            ce = gemv('N', n, j + 1, Vq(q, 0), n, hq, j + 1, 1, -1.0, z, n, 1.0, z, n, w.partial, nullptr, s);
-        }
-        if (ce == cudaSuccess)
-          ce = gemv('T', n, 1, z, n, z, n, 1, 1.0, nullptr, 1, 0.0, w.h + (size_t)(q * 3 + 2) * hs, 1, w.partial,
-                    nullptr, s);
-      }
+      gs(0, j, nullptr, p1, nullptr);
+      gs(1, j, p1, p2, w.h);
+      gs(2, j, p2, pn, w.h + hs);
+      ce = cudaGetLastError();
       if (ce != cudaSuccess) { rc = cuda_fail(ctx, ce, "Gram-Schmidt"); break; }
       {
         LaunchScope ls_(K_REFINE, 0.0, 0.0, s);
-        gmres_step_kernel<<<1, 32, 0, s>>>(nc, j, m, w.h, rtol, w.gm, w.gflags);
+        gmres_step_kernel<<<1, 32, 0, s>>>(nc, j, m, w.h, pn, nblk, rtol, w.gm, w.gflags);
       }
       {
         LaunchScope ls_(K_REFINE, 0.0, 16.0 * n * nc, s);
@@ -961,17 +1077,16 @@ struct Solver {
       gmres_finish_kernel<<<1, 32, 0, s>>>(nc, m, w.gm, w.gflags, w.h);
     }
     GBLU_CK(ctx, cudaGetLastError(), "GMRES finish");
+    {
+      LaunchScope ls_(K_REFINE, 0.0, 0.0, s);
+      gmres_combine_kernel<<<dim3(grid_for(n), nc), 256, 0, s>>>(n, V, ldV, w.h, w.gflags, w.x, n);
+    }
+    GBLU_CK(ctx, cudaGetLastError(), "update");
     std::vector<int> fl(2 * nc);
     GBLU_CK(ctx, cudaMemcpyAsync(fl.data(), w.gflags, 2 * nc * sizeof(int), cudaMemcpyDeviceToHost, s),
             "reading GMRES steps");
     GBLU_CK(ctx, cudaStreamSynchronize(s), "GMRES");
-    for (int q = 0; q < nc; ++q) {
-      its[q] = fl[2 * q + 1];
-      if (its[q] == 0) continue;
-      double* xq = w.x + (size_t)q * n;
-      GBLU_CK(ctx, gemv('N', n, its[q], Vq(q, 0), n, w.h + (size_t)q * hs, its[q], 1, 1.0, xq, n, 1.0, xq, n,
-                        w.partial, nullptr, s), "update");
-    }
+    for (int q = 0; q < nc; ++q) its[q] = fl[2 * q + 1];
     return GBLU_OK;
   }
 };
@@ -1025,7 +1140,8 @@ int32_t refine_solve(gblu_ctx* ctx, gblu_factor* f, char trans, int64_t nrhs, do
     } else {
       GBLU_CK(ctx, cudaMemsetAsync(w.x, 0, (size_t)n * nc * sizeof(double), s), "x0");  // x0 = 0
       for (int it = 0; it <= o.max_iter; ++it) {
-        int32_t e = it == 0 ? S.residual_zero_x(nc, rn.data(), xn.data()) : S.residual(nc, rn.data(), xn.data());
+        int32_t e = it == 0 ? S.residual_zero_x(nc, rn.data(), xn.data())
+                            : S.residual(nc, rn.data(), xn.data(), o.mode == GBLU_REFINE_IR);
         if (e) return e;
         if (it == 0) bn = rn;  // x = 0: r = b
         bool any_active = false;
@@ -1054,14 +1170,10 @@ int32_t refine_solve(gblu_ctx* ctx, gblu_factor* f, char trans, int64_t nrhs, do
           if (e) return e;
           for (int q = 0; q < nc; ++q) st_acc.inner_iterations += its[q];
         } else {
-          e = S.precond(w.r, n, w.r, n, nc);  // d = M^{-1} r (in place), scaled per column
+          unsigned active = 0;
+          for (int q = 0; q < nc; ++q) active |= state[q] == ACTIVE ? 1u << q : 0u;
+          e = S.correct(nc, active);  // x += M^{-1} r
           if (e) return e;
-          for (int q = 0; q < nc; ++q) {
-            if (state[q] != ACTIVE) continue;
-            LaunchScope ls_(K_REFINE, 0.0, 0.0, s);
-            axpby_kernel<<<grid_for(n), 256, 0, s>>>(n, 1.0, w.r + (size_t)q * n, 1.0, w.x + (size_t)q * n);
-          }
-          GBLU_CK(ctx, cudaGetLastError(), "update");
         }
       }
     }
