@@ -185,7 +185,7 @@ size_t factor_arena_bytes(int64_t m, int64_t n, int32_t precision, int device) {
     bytes += align256(tc_work_bytes(n, n / 2 + 64, n / 2 + 64));
     bytes += align256(trsm_inv_bytes(n));
   }
-  bytes += align256(tslu_work_bytes());
+  bytes += align256(std::max(tslu_work_bytes(), genp_work_bytes()));
   if (m == n && n > 0) bytes += align256(getrs_inverse_bytes(n, sizeof(float)));
   if (m == n && n >= 4) bytes += align256((size_t)4 * (n - n % 4) * sizeof(float));  // RBT diagonals
   return bytes;
@@ -365,7 +365,7 @@ int32_t gblu_factor_create(gblu_ctx* ctx, int64_t m, int64_t n, int32_t precisio
       f->rf32.tslu = pe && !strcmp(pe, "tournament");
       if (f->rf32.tslu) f->pivoting = GBLU_PIVOT_TOURNAMENT;
       f->rf32.tslu_work = c;
-      c += align256(tslu_work_bytes());
+      c += align256(std::max(tslu_work_bytes(), genp_work_bytes()));
     }
     // the low-precision solve of a mixed factor is refinement's correction
     // solve: fast (inverted diagonal blocks) by default

@@ -95,8 +95,8 @@ struct GetrfPlan {
   bool tslu = false;
   void* tslu_work = nullptr; // tslu_work_bytes()
   // FP32 working matrix only: no pivoting (the random-butterfly-transformed
-  // factors): each leaf is a no-interchange getf2 of its top block and a
-  // parallel solve below it (tslu.cu), with no laswp
+  // factors): each leaf is a no-interchange LU of its top block and a
+  // parallel solve below it (genp.cu; its work area is tslu_work), with no laswp
   bool nopivot = false;
   // FP32 working matrix of the 16-bit-operand factors only: TRSM base blocks
   // of 65..128 rows solved through inverses of L's diagonal blocks, each
@@ -115,9 +115,14 @@ bool tslu_fits(int64_t rows, int w);
 void tslu_configure(int device);
 cudaError_t tslu_panel_launch(float* A, int64_t lda, int64_t m, int64_t c0, int w, int64_t* ipiv,
                               int64_t* info, void* work, DevScratch* scr, cudaStream_t s);
-// No-pivot leaf (GetrfPlan::nopivot); work: the tslu work area (its ticket).
+// No-pivot leaf (GetrfPlan::nopivot) of w <= kGenpW columns (genp.cu); work:
+// genp_work_bytes().  linv: slot for the inverse of the leaf's L11 (ld kGenpW),
+// or null.
+constexpr int kGenpW = 128;
+size_t genp_work_bytes();
+void genp_configure(int device);
 cudaError_t genp_panel_launch(float* A, int64_t lda, int64_t m, int64_t c0, int w, int64_t* ipiv,
-                              int64_t* info, void* work, cudaStream_t s);
+                              int64_t* info, void* work, float* linv, cudaStream_t s);
 
 // Sub-panel cluster kernel (panel.cu).  panel_sub_width: the leaf width it takes
 // for a leaf of M rows, 0 when it does not take it (or no cluster of 16 CTAs

@@ -1049,6 +1049,7 @@ struct Driver {
     return panel_sub_width<T>(p.m - c0);
   }
   int leaf_width(int64_t c0) const {
+    if (std::is_same<T, float>::value && p.nopivot && p.tslu_work) return kGenpW;
     const int w = sub_width(c0);
     return w > 0 ? w : p.panel_width;
   }
@@ -1059,7 +1060,15 @@ struct Driver {
     if constexpr (std::is_same<T, float>::value) {
       // random-butterfly-transformed factors: no pivot search, no interchanges
       if (p.nopivot && p.tslu_work) {
-        check(genp_panel_launch(p.A, p.lda, p.m, c0, w, p.ipiv, p.info, p.tslu_work, s));
+        // the leaf's kernels leave inverse_slot's inverse of L11 on the way
+        float* linv = nullptr;
+        if (p.trsm_inv && w == kGenpW && c0 + w < p.n && inv_next < p.trsm_inv_slots) {
+          reserve_slots();
+          inv_slot[(size_t)(c0 / 32)] = inv_next;
+          inv_k[(size_t)(c0 / 32)] = kGenpW;
+          linv = p.trsm_inv + (size_t)inv_next++ * kTinvLd * kTinvLd;
+        }
+        check(genp_panel_launch(p.A, p.lda, p.m, c0, w, p.ipiv, p.info, p.tslu_work, linv, s));
         return;
       }
       // low-precision factors: tournament pivoting for the tall leaves
@@ -1163,16 +1172,19 @@ struct Driver {
     check(cudaGetLastError());
   }
 
+  void reserve_slots() {
+    if (!inv_slot.empty()) return;
+    inv_slot.assign((size_t)(p.m / 32 + 2), -1);
+    inv_k.assign(inv_slot.size(), 0);
+  }
+
   // The cached inverse of the k x k diagonal block of L at row r0 (r0 a
   // multiple of 32): computed on first use in this getrf (the block is final
   // once the leaves covering it are done; a later getrf starts a new cache),
   // reused for any order up to k (the leading block of an inverse is the
   // inverse of the leading block).  Returns the slot, or -1 when full.
   int inverse_slot(int64_t r0, int64_t k) {
-    if (inv_slot.empty()) {
-      inv_slot.assign((size_t)(p.m / 32 + 2), -1);
-      inv_k.assign(inv_slot.size(), 0);
-    }
+    reserve_slots();
     const size_t key = (size_t)(r0 / 32);
     if (key >= inv_slot.size()) return -1;
     if (inv_slot[key] >= 0 && inv_k[key] >= k) return inv_slot[key];
@@ -1226,8 +1238,9 @@ struct Driver {
       return;
     }
     int64_t k1 = k / 2;
-    if (p.trsm_inv) {  // halves on 32-row boundaries, so cached blocks recur
-      const int64_t a = (k1 + 31) / 32 * 32;
+    if (p.trsm_inv) {  // halves on 32-row boundaries (leaves', without pivoting), so cached blocks recur
+      const int64_t g = p.nopivot ? kGenpW : 32;
+      const int64_t a = (k1 + g - 1) / g * g;
       if (a < k) k1 = a;
     }
     trsm(r0, k1, bc0, ncols);
@@ -1301,6 +1314,7 @@ void getrf_configure(int device) {
   getrs_configure(device);
   tc_configure(device);
   tslu_configure(device);
+  genp_configure(device);
 }
 
 // GBLU_PANEL=grid|cluster|reg forces one panel kernel (reg: the sub-panel kernel) (where the panel fits
