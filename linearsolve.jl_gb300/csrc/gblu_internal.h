@@ -98,8 +98,8 @@ struct GetrfPlan {
   // factors): each leaf is a no-interchange LU of its top block and a
   // parallel solve below it (genp.cu; its work area is tslu_work), with no laswp
   bool nopivot = false;
-  // FP32 working matrix of the 16-bit-operand factors only: TRSM base blocks
-  // of 65..128 rows solved through inverses of L's diagonal blocks, each
+  // FP32 working matrix of the 16-bit-operand factors only: TRSM bases of
+  // 65..512 rows solved through inverses of L's 128-row diagonal blocks, each
   // computed once per getrf and kept in one of these 128 x 128 slots
   float* trsm_inv = nullptr;
   int trsm_inv_slots = 0;

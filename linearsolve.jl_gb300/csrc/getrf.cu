@@ -578,107 +578,197 @@ constexpr size_t trsm_smem() { return (size_t)KM * KM * sizeof(T); }
 // ---------------------------------------------------------------------------
 // TRSM base blocks of the 16-bit-operand factors (FP32 working matrix; the
 // factors are refinement's preconditioner, not the reference's bit pattern):
-// X = L^-1 of a unit-lower k x k diagonal block (64 < k <= 128) once per
-// getrf, then B := X B as a product, with no dependent chain.
+// X = L^-1 of a unit-lower k x k diagonal block (k <= 128) once per getrf, then
+// products with B, with no dependent chain of columns.
 constexpr int kTinvLd = 128;       // leading dimension of a cached inverse
-constexpr int kTinvApCols = 32;    // B columns per CTA of the product
-constexpr int kTinvApLdB = kTinvLd + 1;
 
-// Warp w of CTA b solves L x = e_j, j = 16 b + w (the TRSM chain, starting
-// at row j: the inverse is lower triangular); column j of X, ld 128.
-__global__ void __launch_bounds__(512)
+// Warp w of CTA b solves L x = e_j, j = 8 b + w (the TRSM chain, starting at row
+// j: the inverse is lower triangular); column j of X, ld 128.  A CTA copies only
+// the columns of L from its first on.  k a multiple of 4, L on 16 bytes.
+constexpr int kTinvCols = 8;       // columns of the inverse per CTA
+constexpr int kTinvLds = kTinvLd + 4;
+__global__ void __launch_bounds__(32 * kTinvCols)
 trsm_inv_kernel(const float* __restrict__ L, int64_t ldl, int k, float* __restrict__ X) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float(*sL)[kTinvLd + 1] = reinterpret_cast<float(*)[kTinvLd + 1]>(smem_raw);  // sL[c][r] = L[r, c]
+  float* sL = reinterpret_cast<float*>(smem_raw);  // sL[c * kTinvLds + r] = L[r, c]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int e = 0; e < kTinvLd * kTinvLd / 512; ++e) {
-    const int idx = e * 512 + (int)threadIdx.x, c = idx / kTinvLd, r = idx % kTinvLd;
-    if (c < k && r > c && r < k) {
-      const unsigned d = (unsigned)__cvta_generic_to_shared(&sL[c][r]);
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(L + r + (int64_t)c * ldl) : "memory");
+  const int j0 = (int)blockIdx.x * kTinvCols;
+  for (int i = threadIdx.x; i < (k - j0) * (kTinvLd / 4); i += 32 * kTinvCols) {
+    const int c = j0 + i / (kTinvLd / 4), r = 4 * (i % (kTinvLd / 4));
+    if (r + 3 > c && r < k) {
+      const unsigned d = (unsigned)__cvta_generic_to_shared(sL + c * kTinvLds + r);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(L + r + (int64_t)c * ldl) : "memory");
     }
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
-  const int j = blockIdx.x * 16 + warp;
+  const int j = j0 + warp;
   if (j >= k) return;
   float v[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) v[q] = lane + 32 * q == j ? 1.f : 0.f;
-  for (int kk = j; kk < k - 1; ++kk) {
-    const int qk = kk >> 5;
-    float src = v[0];
 #pragma unroll
-    for (int q = 1; q < 4; ++q)
-      if (qk == q) src = v[q];
-    const float xk = __shfl_sync(0xffffffffu, src, kk & 31);
+  for (int qk = 0; qk < 4; ++qk) {
+    if (32 * qk + 31 < j) continue;
+    const int end = min(32 * qk + 32, k - 1);
+#pragma unroll 4
+    for (int kk = max(j, 32 * qk); kk < end; ++kk) {
+      const float xk = __shfl_sync(0xffffffffu, v[qk], kk & 31);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (q < qk) continue;
-      const int r = lane + 32 * q;
-      if (r > kk && r < k) v[q] = fmaf(-sL[kk][r], xk, v[q]);
+      for (int q = qk; q < 4; ++q) {
+        const int r = lane + 32 * q;
+        if (r > kk && r < k) v[q] = fmaf(-sL[kk * kTinvLds + r], xk, v[q]);
+      }
     }
   }
 #pragma unroll
   for (int q = 0; q < 4; ++q) X[lane + 32 * q + (int64_t)j * kTinvLd] = lane + 32 * q < k ? v[q] : 0.f;
 }
 
-// B (k x ncols, ldb) := X B with X the cached k x k inverse (ld 128), k a
-// multiple of 4.  CTA: 128 rows x 32 columns; thread (ty, tx) = 4 rows x 4
-// columns, accumulating over the columns kk <= its last row (X is lower
-// triangular).  Each CTA reads its columns of B whole before writing them.
+// B (k x ncols, ldb) := L^-1 B for a unit-lower L of up to four 128-row blocks
+// whose inverses are cached (the last may be shorter; k a multiple of 4): block
+// after block, B_i - sum_j L_ij X_j, then its product with block i's inverse.
+// The columns of B are independent, so a CTA keeps NC of them whole in shared
+// memory and nothing crosses CTAs; 64-column tiles of L and of the inverses
+// stream through a ring of three (32-column ones, twice the barriers: 4 % slower).  Thread (ty, tx): 4 rows x NC / 8 columns with
+// 16-byte loads of both operands.
+// In one launch for a triangle of 512 rows this replaces four products with
+// inverses, two short SIMT updates and a tensor-core update with its operand
+// conversions: BF16 n = 16384 48.1 -> 45.5 ms, FP16 without pivoting n = 6002
+// 6.86 -> 6.11 ms.  Chains of 256 rows: 45.5 and 6.44 ms; of 1024, where the FP32
+// products cost more than the tensor-core update's launches: 47.5 and 6.23 ms.
+constexpr int kTrsmChain = 512;    // rows of a chain
+constexpr int kChainK = 64;        // columns of a tile
+constexpr int kChainStages = 3;
+struct TrsmSlots { const float* p[kTrsmChain / kTinvLd]; };
+
+template <int NC>
 __global__ void __launch_bounds__(256)
-trsm_inv_apply_kernel(const float* __restrict__ X, int k, float* __restrict__ B, int64_t ldb, int64_t ncols) {
+trsm_chain_kernel(const float* __restrict__ L, int64_t ldl, int k, const __grid_constant__ TrsmSlots inv,
+                  float* __restrict__ B, int64_t ldb, int64_t ncols) {
+  constexpr int CPT = NC / 8;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float* sX = reinterpret_cast<float*>(smem_raw);  // sX[kk * 128 + r] = X[r, kk]
-  float* sB = sX + kTinvLd * kTinvLd;             // sB[c * 129 + kk] = B[kk, cb + c]
+  float* sT = reinterpret_cast<float*>(smem_raw);        // [stage][column][128]
+  float* sB = sT + kChainStages * kChainK * kTinvLd;     // sB[c * ldB + row]
+  const int ldB = (k + 31) / 32 * 32 + 4;                // columns on different banks
   const int tid = threadIdx.x, ty = tid >> 3, tx = tid & 7;
-  const int64_t cb = (int64_t)blockIdx.x * kTinvApCols;
-  const int nc = (int)min((int64_t)kTinvApCols, ncols - cb);
-  for (int i = tid; i < k * (kTinvLd / 4); i += 256) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(sX + 4 * i);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(X + 4 * i) : "memory");
+  const int64_t cb = (int64_t)blockIdx.x * NC;
+  const int nc = (int)min((int64_t)NC, ncols - cb);
+  const int nblk = (k + kTinvLd - 1) / kTinvLd;
+  auto cp = [](float* dst, const float* src) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+  };
+  // tiles in order: block row i: L_i0 .. L_i,i-1, then the inverse; (i, j, q) is
+  // the next one to copy
+  int ii = 0, ij = 0, iq = 0, islot = 0;
+  auto issue = [&]() {
+    if (ii < nblk) {
+      const int kb = min(kTinvLd, k - ii * kTinvLd), kc = ij < ii ? kTinvLd : kb;  // rows; columns of this block
+      const int c0 = iq * kChainK, n = min(kChainK, kc - c0);
+      float* dst = sT + islot * kChainK * kTinvLd;
+      if (ij < ii) {
+        const float* src = L + ii * kTinvLd + (int64_t)(ij * kTinvLd + c0) * ldl;
+        for (int e = tid; e < n * (kTinvLd / 4); e += 256) {
+          const int c = e / (kTinvLd / 4), r = 4 * (e % (kTinvLd / 4));
+          if (r < kb) cp(dst + 4 * e, src + r + c * ldl);
+        }
+      } else {
+        const float* src = inv.p[ii] + c0 * kTinvLd;
+        for (int e = tid; e < n * (kTinvLd / 4); e += 256) {
+          const int r = 4 * (e % (kTinvLd / 4));
+          if (r + 3 >= c0) cp(dst + 4 * e, src + 4 * e);  // the rows above are zero
+        }
+      }
+      islot = (islot + 1) % kChainStages;
+      if (c0 + kChainK < kc) ++iq;
+      else { iq = 0; if (ij < ii) ++ij; else { ij = 0; ++ii; } }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int e = tid; e < nc * (k / 4); e += 256) {
+    const int c = e / (k / 4), r = 4 * (e % (k / 4));
+    cp(sB + c * ldB + r, B + r + (cb + c) * ldb);
   }
-  for (int i = tid; i < k * nc; i += 256) {
-    const int c = i / k, kk = i % k;
-    const unsigned d = (unsigned)__cvta_generic_to_shared(sB + c * kTinvApLdB + kk);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(B + kk + (cb + c) * ldb) : "memory");
+#pragma unroll
+  for (int t = 0; t < kChainStages - 1; ++t) issue();
+  float acc[4][CPT];
+  int slot = 0;
+  // acc += sign * tile (columns 0 .. n - 1) * sB rows kbase ..
+  auto product = [&](const float* tile, int kbase, int n, float sign) {
+    const float* bp = sB + tx * ldB + kbase;
+#pragma unroll (NC == 32 ? 2 : 4)
+    for (int kk = 0; kk < n; kk += 4) {
+      float4 b[CPT];
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) b[c] = *reinterpret_cast<const float4*>(bp + 8 * c * ldB + kk);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float4 l = *reinterpret_cast<const float4*>(tile + (kk + q) * kTinvLd + 4 * ty);
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+          const float x = sign * (q == 0 ? b[c].x : q == 1 ? b[c].y : q == 2 ? b[c].z : b[c].w);
+          acc[0][c] = fmaf(l.x, x, acc[0][c]);
+          acc[1][c] = fmaf(l.y, x, acc[1][c]);
+          acc[2][c] = fmaf(l.z, x, acc[2][c]);
+          acc[3][c] = fmaf(l.w, x, acc[3][c]);
+        }
+      }
+    }
+  };
+  auto next_tile = [&]() -> const float* {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kChainStages - 2) : "memory");
+    __syncthreads();  // this tile everywhere, the slot before it free
+    issue();
+    const float* t = sT + slot * kChainK * kTinvLd;
+    slot = (slot + 1) % kChainStages;
+    return t;
+  };
+  for (int i = 0; i < nblk; ++i) {
+    const int kb = min(kTinvLd, k - i * kTinvLd);
+    float* own = sB + tx * ldB + i * kTinvLd + 4 * ty;
+    const bool on = 4 * ty < kb;  // kb is a multiple of 4
+    if (i > 0) {
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) {
+        if (!on) break;
+        const float4 v = *reinterpret_cast<const float4*>(own + 8 * c * ldB);
+        acc[0][c] = v.x; acc[1][c] = v.y; acc[2][c] = v.z; acc[3][c] = v.w;
+      }
+      for (int j = 0; j < i * (kTinvLd / kChainK); ++j) {
+        const float* t = next_tile();
+        if (on) product(t, j * kChainK, kChainK, -1.f);
+      }
+      if (on)  // read by the others after the next tile's barrier
+#pragma unroll
+        for (int c = 0; c < CPT; ++c)
+          *reinterpret_cast<float4*>(own + 8 * c * ldB) = make_float4(acc[0][c], acc[1][c], acc[2][c], acc[3][c]);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) acc[q][c] = 0.f;
+    for (int c0 = 0; c0 < kb; c0 += kChainK) {
+      const float* t = next_tile();
+      // lower triangular: no columns past the thread's last row
+      if (on) product(t, i * kTinvLd + c0, min(kChainK, 4 * ty + 4 - c0), 1.f);
+    }
+    __syncthreads();  // every thread has read block i's right-hand side
+    if (on)
+#pragma unroll
+      for (int c = 0; c < CPT; ++c)
+        *reinterpret_cast<float4*>(own + 8 * c * ldB) = make_float4(acc[0][c], acc[1][c], acc[2][c], acc[3][c]);
   }
-  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) acc[i][c] = 0.f;
-  const int kend = min(k, 4 * ty + 4);
-  const float* bcol = sB + (4 * tx) * kTinvApLdB;
-  for (int kk = 0; kk < kend; ++kk) {
-    const float4 x0 = *reinterpret_cast<const float4*>(sX + kk * kTinvLd + 4 * ty);
-    const float xr[4] = {x0.x, x0.y, x0.z, x0.w};
-    float bv[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) bv[c] = bcol[c * kTinvApLdB + kk];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[i][c] = fmaf(xr[i], bv[c], acc[i][c]);
-  }
-  if (4 * ty >= k) return;
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    if (4 * tx + c >= nc) break;
-    float* dst = B + 4 * ty + (cb + 4 * tx + c) * ldb;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (4 * ty + i < k) dst[i] = acc[i][c];
+  for (int e = tid; e < nc * k; e += 256) {
+    const int c = e / k, r = e % k;
+    B[r + (cb + c) * ldb] = sB[c * ldB + r];
   }
 }
 
-constexpr size_t trsm_inv_smem() { return (size_t)kTinvLd * (kTinvLd + 1) * sizeof(float); }
-constexpr size_t trsm_inv_apply_smem() {
-  return (size_t)kTinvLd * kTinvLd * sizeof(float) + (size_t)kTinvApCols * kTinvApLdB * sizeof(float);
+constexpr size_t trsm_inv_smem() { return (size_t)kTinvLd * kTinvLds * sizeof(float); }
+constexpr size_t trsm_chain_smem(int k, int nc) {
+  return ((size_t)kChainStages * kChainK * kTinvLd + (size_t)nc * ((k + 31) / 32 * 32 + 4)) * sizeof(float);
 }
 
 // ---------------------------------------------------------------------------
@@ -1195,7 +1285,7 @@ struct Driver {
     }
     float* X = p.trsm_inv + (size_t)slot * kTinvLd * kTinvLd;
     LaunchScope ls(K_TRSM, (double)k * k * k / 3.0, ((double)k * k / 2 + (double)k * kTinvLd) * 4.0, s);
-    trsm_inv_kernel<<<(unsigned)((k + 15) / 16), 512, trsm_inv_smem(), s>>>(
+    trsm_inv_kernel<<<(unsigned)((k + kTinvCols - 1) / kTinvCols), 32 * kTinvCols, trsm_inv_smem(), s>>>(
         reinterpret_cast<const float*>(at(r0, r0)), p.lda, (int)k, X);
     check(cudaGetLastError());
     inv_slot[key] = slot;
@@ -1203,21 +1293,36 @@ struct Driver {
     return slot;
   }
 
+  // The chain of inverses for a triangle of up to kTrsmChain rows; false when
+  // the matrix is not aligned or the inverse cache is full.  Columns a CTA: more
+  // read the tiles of L less often, fewer leave no SM idle; the widest that
+  // gives half the SMs a CTA (32 only from one CTA an SM on: 2 % slower).
+  bool trsm_chain(int64_t r0, int k, int64_t bc0, int64_t ncols) {
+    if (((reinterpret_cast<uintptr_t>(at(r0, r0)) | reinterpret_cast<uintptr_t>(at(r0, bc0)) | (uintptr_t)(p.lda * 4)) & 15) != 0)
+      return false;  // its copies are of 16 bytes
+    TrsmSlots sl{};
+    for (int i = 0; i * kTinvLd < k; ++i) {
+      const int slot = inverse_slot(r0 + i * kTinvLd, std::min(kTinvLd, k - i * kTinvLd));
+      if (slot < 0) return false;
+      sl.p[i] = p.trsm_inv + (size_t)slot * kTinvLd * kTinvLd;
+    }
+    const int sms = device_info(device).num_sms;
+    const int nc = ncols >= 16 * (int64_t)sms ? 32 : ncols >= 8 * (int64_t)sms ? 16 : 8;
+    const unsigned grid = (unsigned)((ncols + nc - 1) / nc);
+    LaunchScope ls(K_TRSM, (double)k * k * ncols, (2.0 * k * ncols + (double)k * k) * 4.0, s);
+    auto* kern = nc == 32 ? trsm_chain_kernel<32> : nc == 16 ? trsm_chain_kernel<16> : trsm_chain_kernel<8>;
+    kern<<<grid, 256, trsm_chain_smem(k, nc), s>>>(reinterpret_cast<const float*>(at(r0, r0)), p.lda, k, sl,
+                                                   reinterpret_cast<float*>(at(r0, bc0)), p.lda, ncols);
+    check(cudaGetLastError());
+    return true;
+  }
+
   // B (k x ncols at (r0, bc0)) := L \ B, L unit lower at (r0, r0) of size k.
   void trsm(int64_t r0, int64_t k, int64_t bc0, int64_t ncols) {
     if (k <= 0 || ncols <= 0) return;
     if constexpr (std::is_same<T, float>::value) {
-      if (p.trsm_inv && k > 64 && k <= kTinvLd && k % 4 == 0 && r0 % 32 == 0) {
-        const int slot = inverse_slot(r0, k);
-        if (slot >= 0) {
-          LaunchScope ls(K_TRSM, 2.0 * k * k * ncols / 2.0, (2.0 * k * ncols + (double)k * k) * 4.0, s);
-          trsm_inv_apply_kernel<<<(unsigned)((ncols + kTinvApCols - 1) / kTinvApCols), 256,
-                                  trsm_inv_apply_smem(), s>>>(p.trsm_inv + (size_t)slot * kTinvLd * kTinvLd,
-                                                              (int)k, at(r0, bc0), p.lda, ncols);
-          check(cudaGetLastError());
-          return;
-        }
-      }
+      if (p.trsm_inv && k > 64 && k <= kTrsmChain && k % 4 == 0 && r0 % 32 == 0 && trsm_chain(r0, (int)k, bc0, ncols))
+        return;
     }
     if (k <= p.trsm_base && k <= kTrsmMax) {
       const DeviceInfo& di = device_info(device);
@@ -1238,8 +1343,10 @@ struct Driver {
       return;
     }
     int64_t k1 = k / 2;
-    if (p.trsm_inv) {  // halves on 32-row boundaries (leaves', without pivoting), so cached blocks recur
-      const int64_t g = p.nopivot ? kGenpW : 32;
+    // halves of whole blocks, so the cached inverses recur; of 32 rows where a
+    // chain found no slots
+    if (p.trsm_inv) {
+      const int64_t g = k > kTrsmChain ? kTinvLd : 32;
       const int64_t a = (k1 + g - 1) / g * g;
       if (a < k) k1 = a;
     }
@@ -1255,6 +1362,9 @@ struct Driver {
       return;
     }
     int64_t w1 = ((w / 2 + wb - 1) / wb) * wb;
+    // whole blocks of the TRSM inverse cache (the leaf widths divide them), so
+    // every triangle's blocks are the same ones
+    if (p.trsm_inv && w1 > kTinvLd) w1 = (w1 + kTinvLd - 1) / kTinvLd * kTinvLd;
     if (w1 >= w) w1 = w - wb;
     rec(c0, w1);
     const int64_t c1 = c0 + w1, w2 = w - w1;
@@ -1291,8 +1401,12 @@ size_t trsm_inv_bytes(int64_t n) {
 
 void getrf_configure(int device) {
   cudaFuncSetAttribute(trsm_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_inv_smem());
-  cudaFuncSetAttribute(trsm_inv_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)trsm_inv_apply_smem());
+  cudaFuncSetAttribute(trsm_chain_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)trsm_chain_smem(kTrsmChain, 32));
+  cudaFuncSetAttribute(trsm_chain_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)trsm_chain_smem(kTrsmChain, 16));
+  cudaFuncSetAttribute(trsm_chain_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)trsm_chain_smem(kTrsmChain, 8));
   const DeviceInfo& di = device_info(device);
   const int cap = (int)std::min<size_t>(di.smem_optin, 200 * 1024);
   cudaFuncSetAttribute(panel_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
