@@ -1005,11 +1005,11 @@ def run_kernel_case(args) -> int:
     """One small invocation of a group of kernels, for ncu (no timing, no
     JSON line): operands larger than L2 so DRAM counters mean something.
       gemm_bf16 / gemm_fp16  C -= A B, M = N = K = 4096 through gblu_gemm_update
-                             (conv_a / col_scale / conv_b + tc_gemm_kernel)
+                             (conv_ab_kernel + tc_gemm_kernel)
       gemm_fp32              the same on the FP32 SIMT path (gemm_sub_f32_rb_kernel)
       refine                 FP32 factor of n = 6144 (convert_f64_f32, umax) and refined
                              solves of 4 RHS, IR then GMRES-IR (gemv partial / reduce,
-                             colmax, pow2_scales, scale_to_f32, update_from_f32, axpby)
+                             colmax, scale_to_f32, correct, update_from_f32, gmres_gs / combine)
       perm                   LAPACK-shaped dgetrs with host factors and pivots, n = 8192
                              (upload_ipiv_check_kernel, perm_from_ipiv_kernel)
       mixed_bf16             the mixed suite's BF16 solve set, n = 16384, 4 RHS, run twice
@@ -1017,7 +1017,7 @@ def run_kernel_case(args) -> int:
       mixed_bf16_rbt         the same with no pivoting after the random butterfly transform
       step_fp64              two steps of the headline workload (n = 8192, 1 getrf + 16 getrs)
       getrs_fast             the same factorization, then 8 single-RHS solves in fast mode
-      helpers                n = 6144: BF16 factor (trsm_inv / trsm_inv_apply, prepare and
+      helpers                n = 6144: BF16 factor (trsm_inv / trsm_chain, prepare and
                              its reduction, diag_inverse of the fast solve) with a GMRES-IR
                              solve (gmres_begin / step / scale / finish); the same factor
                              with tournament pivoting (tslu_select / tslu_apply); an FP64
@@ -1025,7 +1025,7 @@ def run_kernel_case(args) -> int:
                              FP64 n = 4096 factor on the shared-memory cluster panel
                              (panel_cluster_kernel, forced with GBLU_PANEL=cluster); a BF16
                              factor with no pivoting after the butterfly transform
-                             (rbt_matrix, genp_panel, rbt_vec)"""
+                             (rbt_matrix, genp_top / genp_below, rbt_vec)"""
     pkg = load_pkg()
     _, _, local = dist_env()
     ctx = pkg.Context(local)

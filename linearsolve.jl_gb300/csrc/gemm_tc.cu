@@ -317,78 +317,80 @@ __device__ __forceinline__ uint2 pack4(float a, float b, float c, float d) {
   return make_uint2(lo, hi);
 }
 
-// A (M x K, column-major, lda) -> Ah (M rows of K, row-major, ldh, ldh a
-// multiple of 8): 64 x 64 tiles through shared memory; a warp reads 64
-// consecutive rows of a column and each thread writes 4 consecutive k of a
-// row as one 8-byte store.
+// Both operands in one launch: a launch of its own for each, and for the FP16
+// scales, cost more than the conversion of most updates (BF16 n = 16384 45.5 ->
+// 44.7 ms, FP16 without pivoting n = 6002 6.11 -> 5.74 ms).
+//   CTAs 0 .. b_ctas - 1: B (K x N, column-major, ldb) -> Bh (N rows of K, ldh a
+//     multiple of 8).  A column of B is a row of Bh: 64 threads a column convert
+//     4 consecutive k with one 8-byte store, 4 columns per CTA.  FP16: the column
+//     is scaled by a power of two that takes its maximum to [2^14, 2^15) first
+//     (inv_scale: the inverse, for the epilogue).
+//   The others: A (M x K, column-major, lda) -> Ah (M rows of K): 64 x 64 tiles
+//     through shared memory; a warp reads 64 consecutive rows of a column and
+//     each thread writes 4 consecutive k of a row as one 8-byte store.
 template <typename H>
 __global__ void __launch_bounds__(256)
-conv_a_kernel(int M, int K, const float* __restrict__ A, int64_t lda, H* __restrict__ Ah, int64_t ldh) {
+conv_ab_kernel(int M, int N, int K, const float* __restrict__ A, int64_t lda, const float* __restrict__ B,
+               int64_t ldb, H* __restrict__ Ah, H* __restrict__ Bh, int64_t ldh, int b_ctas, int k_tiles,
+               float* __restrict__ inv_scale) {
+  constexpr bool kScale = !std::is_same<H, __nv_bfloat16>::value;
   __shared__ float t[64][65];  // t[k][m]
-  const int k0 = blockIdx.x * 64, m0 = blockIdx.y * 64;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int kk = warp; kk < 64; kk += 8) {
-    const int k = k0 + kk, m = m0 + 2 * lane;
-    float v0 = 0.f, v1 = 0.f;
-    if (k < K) {
-      const float* src = A + (int64_t)k * lda;
-      if (m < M) v0 = src[m];
-      if (m + 1 < M) v1 = src[m + 1];
+  if ((int)blockIdx.x < b_ctas) {
+    const int n = (int)blockIdx.x * 4 + (threadIdx.x >> 6);
+    const float* col = B + (int64_t)n * ldb;
+    float s = 1.f;
+    if constexpr (kScale) {
+      float mx = 0.f;
+      if (n < N)
+        for (int k = threadIdx.x & 63; k < K; k += 64) mx = fmaxf(mx, fabsf(col[k]));
+      for (int off = 16; off; off >>= 1) mx = fmaxf(mx, __shfl_down_sync(0xffffffffu, mx, off));
+      if (lane == 0) t[0][warp] = mx;
+      __syncthreads();
+      const float m = fmaxf(t[0][warp & ~1], t[0][warp | 1]);
+      int e = 0;
+      if (m > 0.f && isfinite(m)) e = ilogbf(m) - 14;  // m * 2^-e in [2^14, 2^15)
+      e = max(-120, min(120, e));
+      s = ldexpf(1.f, -e);
+      if (n < N && (threadIdx.x & 63) == 0) inv_scale[n] = ldexpf(1.f, e);
     }
-    t[kk][2 * lane] = v0;
-    t[kk][2 * lane + 1] = v1;
-  }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < 64 * 16; idx += 256) {
-    const int mm = idx >> 4, q = idx & 15;  // row of the tile, pack of 4 k
-    const int m = m0 + mm, k = k0 + 4 * q;
-    if (m < M && k < ldh) {  // k < ldh implies k + 4 <= ldh (both multiples of 4)
+    if (n >= N) return;
+    for (int64_t k = 4 * (threadIdx.x & 63); k < ldh; k += 256) {
       float v[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] = (k + i < K) ? t[4 * q + i][mm] : 0.f;
-      *reinterpret_cast<uint2*>(Ah + (int64_t)m * ldh + k) = pack4<H>(v[0], v[1], v[2], v[3]);
+      for (int i = 0; i < 4; ++i) v[i] = (k + i < K) ? col[k + i] * s : 0.f;
+      *reinterpret_cast<uint2*>(Bh + (int64_t)n * ldh + k) = pack4<H>(v[0], v[1], v[2], v[3]);
+    }
+    return;
+  }
+  const int tile = (int)blockIdx.x - b_ctas;
+  const int k0 = tile % k_tiles * 64, m0 = tile / k_tiles * 64;
+  float v0[8], v1[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int k = k0 + warp + 8 * j, m = m0 + 2 * lane;
+    v0[j] = v1[j] = 0.f;
+    if (k < K) {
+      const float* src = A + (int64_t)k * lda;
+      if (m < M) v0[j] = src[m];
+      if (m + 1 < M) v1[j] = src[m + 1];
     }
   }
-}
-
-// B (K x N, column-major, ldb) -> Bh (N rows of K, ldh a multiple of 8), row n
-// scaled by scale[n]: a column of B is a row of Bh, so each thread converts
-// 4 consecutive k with one 8-byte store; 4 columns per CTA.
-template <typename H>
-__global__ void __launch_bounds__(256)
-conv_b_kernel(int K, int N, const float* __restrict__ B, int64_t ldb, H* __restrict__ Bh, int64_t ldh,
-              const float* __restrict__ scale) {
-  const int n = blockIdx.x * 4 + (threadIdx.x >> 6);
-  if (n >= N) return;
-  const float s = scale ? scale[n] : 1.f;
-  const float* col = B + (int64_t)n * ldb;
-  for (int64_t k = 4 * (threadIdx.x & 63); k < ldh; k += 256) {
-    float v[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = (k + i < K) ? col[k + i] * s : 0.f;
-    *reinterpret_cast<uint2*>(Bh + (int64_t)n * ldh + k) = pack4<H>(v[0], v[1], v[2], v[3]);
+  for (int j = 0; j < 8; ++j) {
+    t[warp + 8 * j][2 * lane] = v0[j];
+    t[warp + 8 * j][2 * lane + 1] = v1[j];
   }
-}
-
-// Per-column power-of-two scale for FP16: max |B[:,n]| -> [2^14, 2^15).
-__global__ void col_scale_kernel(int K, int N, const float* __restrict__ B, int64_t ldb,
-                                 float* __restrict__ scale, float* __restrict__ inv_scale) {
-  __shared__ float red[8];
-  const int n = blockIdx.x;
-  if (n >= N) return;
-  float mx = 0.f;
-  for (int k = threadIdx.x; k < K; k += blockDim.x) mx = fmaxf(mx, fabsf(B[(int64_t)k + (int64_t)n * ldb]));
-  for (int off = 16; off; off >>= 1) mx = fmaxf(mx, __shfl_down_sync(0xffffffffu, mx, off));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float m = 0.f;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = fmaxf(m, red[w]);
-    int e = 0;
-    if (m > 0.f && isfinite(m)) e = ilogbf(m) - 14;  // m * 2^-e in [2^14, 2^15)
-    e = max(-120, min(120, e));
-    scale[n] = ldexpf(1.f, -e);
-    inv_scale[n] = ldexpf(1.f, e);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int idx = threadIdx.x + 256 * j;
+    const int mm = idx >> 4, q = idx & 15;  // row of the tile, pack of 4 k
+    const int m = m0 + mm, k = k0 + 4 * q;
+    if (m < M && k < ldh)  // k < ldh implies k + 4 <= ldh (both multiples of 4)
+      // columns past K were stored as zeros
+      *reinterpret_cast<uint2*>(Ah + (int64_t)m * ldh + k) =
+          pack4<H>(t[4 * q][mm], t[4 * q + 1][mm], t[4 * q + 2][mm], t[4 * q + 3][mm]);
   }
 }
 
@@ -458,32 +460,23 @@ cudaError_t tc_gemm_sub(int mode, int64_t M, int64_t N, int64_t K, const float* 
   unsigned char* w = reinterpret_cast<unsigned char*>(work);
   void* Ah = w;
   void* Bh = w + (((size_t)M * Kp * 2 + 255) & ~size_t(255));
-  float* scale = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(Bh) +
-                                          (((size_t)N * Kp * 2 + 255) & ~size_t(255)));
-  float* inv_scale = scale + N;
+  float* inv_scale = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(Bh) +
+                                              (((size_t)N * Kp * 2 + 255) & ~size_t(255)));
   {
+    const int64_t k_tiles = (Kp + 63) / 64, b_ctas = (N + 3) / 4, ctas = b_ctas + k_tiles * ((M + 63) / 64);
+    if (ctas > INT32_MAX) return cudaErrorInvalidValue;
     LaunchScope ls(K_GEMM, 0.0, (double)(M * K + K * N) * 6.0, s);
-    dim3 ga((unsigned)((Kp + 63) / 64), (unsigned)((M + 63) / 64));
     if (bf16)
-      tc::conv_a_kernel<__nv_bfloat16><<<ga, 256, 0, s>>>((int)M, (int)K, A, lda,
-                                                          reinterpret_cast<__nv_bfloat16*>(Ah), Kp);
+      tc::conv_ab_kernel<__nv_bfloat16><<<(unsigned)ctas, 256, 0, s>>>(
+          (int)M, (int)N, (int)K, A, lda, B, ldb, reinterpret_cast<__nv_bfloat16*>(Ah),
+          reinterpret_cast<__nv_bfloat16*>(Bh), Kp, (int)b_ctas, (int)k_tiles, nullptr);
     else
-      tc::conv_a_kernel<__half><<<ga, 256, 0, s>>>((int)M, (int)K, A, lda, reinterpret_cast<__half*>(Ah), Kp);
+      tc::conv_ab_kernel<__half><<<(unsigned)ctas, 256, 0, s>>>((int)M, (int)N, (int)K, A, lda, B, ldb,
+                                                                reinterpret_cast<__half*>(Ah),
+                                                                reinterpret_cast<__half*>(Bh), Kp, (int)b_ctas,
+                                                                (int)k_tiles, inv_scale);
   }
   cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  {
-    LaunchScope ls(K_GEMM, 0.0, (double)(K * N) * 6.0, s);
-    if (bf16) {
-      tc::conv_b_kernel<__nv_bfloat16><<<(unsigned)((N + 3) / 4), 256, 0, s>>>(
-          (int)K, (int)N, B, ldb, reinterpret_cast<__nv_bfloat16*>(Bh), Kp, nullptr);
-    } else {
-      tc::col_scale_kernel<<<(unsigned)N, 256, 0, s>>>((int)K, (int)N, B, ldb, scale, inv_scale);
-      tc::conv_b_kernel<__half><<<(unsigned)((N + 3) / 4), 256, 0, s>>>((int)K, (int)N, B, ldb,
-                                                             reinterpret_cast<__half*>(Bh), Kp, scale);
-    }
-  }
-  e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   // 128 x 256 tiles when they still cover the SMs, else 128 x 128
   int device = 0;
