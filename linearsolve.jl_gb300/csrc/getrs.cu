@@ -35,7 +35,12 @@ constexpr int kTS = kGetrsTile;  // block-row height == tile width
 // InvL_bb, InvU_bb, InvL_bb L_{b,b-1}, InvU_bb U_{b,b+1}
 constexpr int kInvSlots = 4;
 
-constexpr int kSweepThreads = 128;  // all issue copies; threads 0..63 own one row each
+constexpr int kSweepThreads = 128;  // exact sweeps: all issue copies; threads 0..63 own one row each
+// Threads per row of the fast sweeps, each taking its share of a tile's columns:
+// FP32 products are bound by their instructions' latency, FP64 ones by the SM's
+// FP64 pipe, where more threads gain nothing.
+template <typename T>
+constexpr int kFastSplit = sizeof(T) == 4 ? 4 : 2;
 constexpr int kStages = 3;          // tiles in flight per CTA
 
 template <typename T>
@@ -58,28 +63,32 @@ __host__ __device__ constexpr int tile_ld() { return kTS + 16 / (int)sizeof(T); 
 
 // Issue the copies of tile element (r, c) = op(LU)[r0 + r, c0 + c] into t[c][r];
 // 'N': LU[r0+r + (c0+c)*lda] (contiguous in r), 'T': LU[c0+c + (r0+r)*lda]
-// (contiguous in c).  Elements outside nr x nc are zero-filled.  A full 'N'
-// tile of a 16-byte-aligned matrix (vec16) moves in 16-byte copies, each
-// thread walking a fixed row slice across every (kSweepThreads / 16-byte
-// copies per column)-th column.
-template <typename T, bool TRANS>
+// (contiguous in c).  Elements outside nr x nc are zero-filled, not read.  An
+// 'N' tile of a 16-byte-aligned matrix (vec16) moves in 16-byte copies, each
+// thread walking a fixed row slice across every (THREADS / 16-byte copies per
+// column)-th column; a ragged tile's copies take fewer source bytes.  (With
+// element copies for those, the last block row, which has the most tiles, came
+// 15 us after the others at n = 3000.)
+template <typename T, bool TRANS, int THREADS = kSweepThreads>
 __device__ __forceinline__ void issue_tile(T (*t)[tile_ld<T>()], const T* __restrict__ LU, int64_t lda,
                                            int64_t r0, int64_t c0, int nr, int nc, bool vec16) {
-  if (!TRANS && vec16 && nr == kTS && nc == kTS) {
+  if (!TRANS && vec16) {
     constexpr int V = 16 / (int)sizeof(T);    // elements per copy
     constexpr int CPC = kTS / V;              // copies per column
-    constexpr int CSTEP = kSweepThreads / CPC;  // columns per pass
+    constexpr int CSTEP = THREADS / CPC;  // columns per pass
     const int cl = (int)threadIdx.x / CPC, rv = ((int)threadIdx.x % CPC) * V;
     const T* src = LU + (r0 + rv) + (c0 + cl) * lda;
+    const int sz = min(V, max(nr - rv, 0)) * (int)sizeof(T);
 #pragma unroll
     for (int c = cl; c < kTS; c += CSTEP, src += CSTEP * lda) {
       const unsigned d = (unsigned)__cvta_generic_to_shared(&t[c][rv]);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+      const int n = c < nc ? sz : 0;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(n ? src : LU), "r"(n) : "memory");
     }
     return;
   }
 #pragma unroll 8
-  for (int idx = threadIdx.x; idx < kTS * kTS; idx += kSweepThreads) {
+  for (int idx = threadIdx.x; idx < kTS * kTS; idx += THREADS) {
     const int a = idx >> 6, b = idx & 63;  // b runs along the contiguous direction
     const int r = TRANS ? a : b, c = TRANS ? b : a;
     const bool ok = r < nr && c < nc;
@@ -368,20 +377,56 @@ solve_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32
   }
 }
 
+__device__ __forceinline__ unsigned cluster_ctarank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ unsigned cluster_nctarank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+__device__ __forceinline__ int ld_cluster(uint32_t a) {
+  int v;
+  asm volatile("ld.relaxed.cluster.shared::cluster.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_cluster(uint32_t a, float v) {
+  asm volatile("st.relaxed.cluster.shared::cluster.b32 [%0], %1;" ::"r"(a), "r"(__float_as_int(v)) : "memory");
+}
+__device__ __forceinline__ void st_cluster(uint32_t a, double v) {
+  asm volatile("st.relaxed.cluster.shared::cluster.b64 [%0], %1;" ::"r"(a), "l"(__double_as_longlong(v)) : "memory");
+}
+
 // Fast sweeps.  'N': block row i's solution is x_i = d_i - M_i x_p, where x_p
 // is the block row just before it in the sweep, M_i its coupling (fold_kernel)
 // and d_i = Inv_ii (b_i - the products with every earlier block row but x_p):
 // d_i is computed while x_p is still being solved, so only the 64 x 64
 // product M_i x_p lies on the wavefront's critical path.  'T' has no coupling:
-// x_i = op(Inv_ii) (b_i - every product).  Two threads per
-// row, each taking half of every tile's columns with four independent
+// x_i = op(Inv_ii) (b_i - every product).  H threads per
+// row, each taking its share of every tile's columns with four independent
 // partial sums, combined through shared memory.  Tile order per block row:
 // the earlier off-diagonal blocks (but the last, in sweep order, for 'N'),
-// Inv_ii, then M_i.  NR right-hand sides per CTA: one in FP64 (a warp issues
-// an FP64 instruction per 68 cycles, so more would add up along the chain),
-// up to eight in FP32.  Backward-error accurate, not bit-exact.
+// Inv_ii, then M_i, whose share each thread holds in registers before x_p comes.
+// NR right-hand sides per CTA: one in FP64 (a warp issues an FP64 instruction per
+// 68 cycles, so more would add up along the chain), up to two in FP32, more going
+// to CTAs of their own.
+// The CTAs of a cluster are consecutive block rows of the same right-hand sides:
+// a solution goes straight to the shared memory of the next two, which poll it
+// there like the published values (sentinel until then) without the trip through
+// L2 (a store and a load, 1100 cycles).  A block row then takes 0.8 us, of which
+// d_i after x_{i-2} is most (1250 cycles: two products and their sums).
+// FP32 factors, n = 3000, four right-hand sides, one sweep: 79 us with four
+// right-hand sides and two threads a row in a CTA and no clusters, 64 with two
+// right-hand sides a CTA, 58 with four threads a row, 54 with one neighbour
+// pushed to, 46 with two and ragged tiles in 16-byte copies.
+// Backward-error accurate, not bit-exact.
 template <typename T, int NR, bool TRANS, bool FWD>
-__global__ void __launch_bounds__(kSweepThreads)
+__global__ void __launch_bounds__(kTS* kFastSplit<T>)
 fast_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32_t* __restrict__ perm,
                   const T* __restrict__ In, int64_t ldi, T* __restrict__ Y, int64_t ldy,
                   T* __restrict__ Out, int64_t ldo, int nrhs, DevScratch* __restrict__ scr,
@@ -389,16 +434,27 @@ fast_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32_
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T(*tiles)[kTS][tile_ld<T>()] = reinterpret_cast<T(*)[kTS][tile_ld<T>()]>(smem_raw);
   __shared__ T sx[kTS][NR];
-  __shared__ T part[2][kTS][NR];
+  constexpr int H = kFastSplit<T>, Q = kTS / H, kThreads = kTS * H;
+  static_assert(NR <= H, "thread (r, q) finishes row r of right-hand side q");
+  __shared__ T part[H][kTS][NR];
+  __shared__ T s_lx[2][kTS][NR];  // the block rows one and two before this one, pushed by their CTAs
   __shared__ int s_ticket;
+  const int rank = (int)cluster_ctarank(), cs = (int)cluster_nctarank();
   const bool vec16 = ((reinterpret_cast<uintptr_t>(LU) | (uintptr_t)(lda * (int64_t)sizeof(T))) & 15) == 0;
   const int nblk = (int)((n + kTS - 1) / kTS);
   constexpr bool kCouple = !TRANS;
   constexpr bool kUnit = FWD != TRANS;
-  if (threadIdx.x == 0) s_ticket = (int)atomicAdd(&scr->ticket, 1u);
-  __syncthreads();
-  const int groups = (nrhs + NR - 1) / NR;  // CTAs per block row
-  const int ord = s_ticket / groups, q0 = (s_ticket - ord * groups) * NR;
+  if (threadIdx.x == 0 && rank == 0) s_ticket = (int)atomicAdd(&scr->ticket, 1u);  // one a cluster
+  for (int e = threadIdx.x; e < 2 * kTS * NR; e += kThreads)
+    (&s_lx[0][0][0])[e] = SweepBits<T>::as_t(SweepBits<T>::kSentinel);
+  cluster_sync_all();  // every CTA of the cluster runs and has its s_lx
+  const int ticket = ld_cluster(pan_mapa(pan_saddr(&s_ticket), 0));
+  const int groups = (nrhs + NR - 1) / NR;  // clusters per cs block rows
+  const int ord = ticket / groups * cs + rank, q0 = ticket % groups * NR;
+  if (ord >= nblk) {  // the last cluster's spare CTAs
+    cluster_sync_all();
+    return;
+  }
   const int blk = FWD ? ord : nblk - 1 - ord;
   nrhs = min(NR, nrhs - q0);
   if (In) In += q0 * ldi;
@@ -417,11 +473,11 @@ fast_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32_
   auto issue = [&](int t) {
     if (t < nlead) {
       const int64_t c0 = (int64_t)col_block(t) * kTS;
-      issue_tile<T, TRANS>(tiles[t % kStages], LU, lda, r0, c0, nr, (int)min((int64_t)kTS, n - c0), vec16);
+      issue_tile<T, TRANS, kThreads>(tiles[t % kStages], LU, lda, r0, c0, nr, (int)min((int64_t)kTS, n - c0), vec16);
     } else {
       const bool coupling = t > nlead;
       const int slot = (coupling ? 2 : 0) + (kUnit ? 0 : 1);  // L's, U's
-      issue_tile<T, TRANS>(tiles[t % kStages], inv + ((int64_t)blk * kInvSlots + slot) * (kTS * kTS), kTS, 0, 0,
+      issue_tile<T, TRANS, kThreads>(tiles[t % kStages], inv + ((int64_t)blk * kInvSlots + slot) * (kTS * kTS), kTS, 0, 0,
                            nr, coupling ? pnc : nr, true);
     }
   };
@@ -434,9 +490,7 @@ fast_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32_
 #pragma unroll
     for (int q = 0; q < NR; ++q)
       if (q < nrhs) a[0][q] = FWD ? In[(TRANS ? r0 + r : (int64_t)perm[r0 + r]) + q * ldi] : Y[(r0 + r) + q * ldy];
-  T d[NR];
-#pragma unroll
-  for (int q = 0; q < NR; ++q) d[q] = T(0);
+  T d = T(0);  // thread (r, q): row r of right-hand side q
 #pragma unroll
   for (int t = 0; t < kStages - 1; ++t) {
     if (t < ntiles) issue(t);
@@ -444,7 +498,7 @@ fast_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32_
   }
   // solution values of the next block needed, fetched one step ahead
   using UB = typename SweepBits<T>::U;
-  constexpr int KP = (kTS * NR + kSweepThreads - 1) / kSweepThreads;
+  constexpr int KP = (kTS * NR + kThreads - 1) / kThreads;
   UB pre[KP];
   auto src_of = [&](int cb, int c, int q) -> const T* {
     const int64_t c0 = (int64_t)cb * kTS;
@@ -454,43 +508,54 @@ fast_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32_
     const int nc = (int)min((int64_t)kTS, n - (int64_t)cb * kTS);
 #pragma unroll
     for (int k = 0; k < KP; ++k) {
-      const int idx = tid + k * kSweepThreads;
+      const int idx = tid + k * kThreads;
       const int c = idx / NR, q = idx - c * NR;
       pre[k] = (idx < kTS * NR && q < nrhs && c < nc) ? SweepBits<T>::load(src_of(cb, c, q)) : UB(0);
     }
   };
   auto fill_sx = [&](int cb) -> int {
     const int nc = (int)min((int64_t)kTS, n - (int64_t)cb * kTS);
+    const int back = abs(pcb - cb);  // 0: the block row just before
+    const bool pushed = back < 2 && rank > back;
     int ok = 1;
 #pragma unroll
     for (int k = 0; k < KP; ++k) {
-      const int idx = tid + k * kSweepThreads;
+      const int idx = tid + k * kThreads;
       if (idx >= kTS * NR) continue;
       const int c = idx / NR, q = idx - c * NR;
       T v = T(0);
       if (q < nrhs && c < nc) {
-        if (pre[k] != SweepBits<T>::kSentinel) v = SweepBits<T>::as_t(pre[k]);
+        if (pushed) v = smem_value(&s_lx[back][c][q], scr);
+        else if (pre[k] != SweepBits<T>::kSentinel) v = SweepBits<T>::as_t(pre[k]);
         else if (!poll_value(src_of(cb, c, q), scr, &v)) ok = 0;
       }
       sx[c][q] = v;
     }
     return ok;
   };
-  // this thread's half of a tile's columns times sx, added to (sign -1) or
+  // this thread's share of a tile's columns times sx, added to (sign -1) or
   // into fresh sums (sign +1)
-  auto half_product = [&](T(*tile)[tile_ld<T>()], T(&y)[4][NR], T sign) {
-#pragma unroll 2
-    for (int c = 32 * h; c < 32 * h + 32; c += 4) {
-      const T m0 = sign * tile[c][r], m1 = sign * tile[c + 1][r], m2 = sign * tile[c + 2][r],
-              m3 = sign * tile[c + 3][r];
+  auto share_product = [&](T(*tile)[tile_ld<T>()], T(&y)[4][NR], T sign) {
+#pragma unroll 4
+    for (int c = Q * h; c < Q * h + Q; c += 4)
 #pragma unroll
-      for (int q = 0; q < NR; ++q) {
-        y[0][q] = fma(m0, sx[c][q], y[0][q]);
-        y[1][q] = fma(m1, sx[c + 1][q], y[1][q]);
-        y[2][q] = fma(m2, sx[c + 2][q], y[2][q]);
-        y[3][q] = fma(m3, sx[c + 3][q], y[3][q]);
+      for (int j = 0; j < 4; ++j) {
+        const T m = sign * tile[c + j][r];
+#pragma unroll
+        for (int q = 0; q < NR; ++q) y[j][q] = fma(m, sx[c + j][q], y[j][q]);
       }
-    }
+  };
+  // this thread's sums over its share to `part`; then row r's whole sum of
+  // right-hand side h
+  auto put_part = [&](T(&y)[4][NR]) {
+#pragma unroll
+    for (int q = 0; q < NR; ++q) part[h][r][q] = (y[0][q] + y[1][q]) + (y[2][q] + y[3][q]);
+  };
+  auto total = [&]() {
+    T t = part[0][r][h];
+#pragma unroll
+    for (int k = 1; k < H; ++k) t += part[k][r][h];
+    return t;
   };
   if (nlead > 0) prefetch(col_block(0));
   else if (kCouple && noff > 0) prefetch(pcb);
@@ -502,65 +567,52 @@ fast_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32_
     T(*tile)[tile_ld<T>()] = tiles[t % kStages];
     if (t < nlead) {  // an earlier off-diagonal block: b -= L_ij x_j
       const int ok = fill_sx(col_block(t));
-      if (!__syncthreads_and(ok)) {
-        cp_async_wait<0>();  // no copy may land after the CTA has left
-        return;
-      }
+      if (!__syncthreads_and(ok)) break;  // the error word is set
       if (t + 1 < nlead) prefetch(col_block(t + 1));
       else if (kCouple) prefetch(pcb);
-      half_product(tile, a, T(-1));
+      share_product(tile, a, T(-1));
       continue;
-    }
-    if (t == nlead) {  // d = Inv_ii (right-hand side so far)
-#pragma unroll
-      for (int q = 0; q < NR; ++q) part[h][r][q] = (a[0][q] + a[1][q]) + (a[2][q] + a[3][q]);
-      __syncthreads();
-      if (h == 0)
-#pragma unroll
-        for (int q = 0; q < NR; ++q) sx[r][q] = valid ? part[0][r][q] + part[1][r][q] : T(0);
-      __syncthreads();
-      T y[4][NR];
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int q = 0; q < NR; ++q) y[j][q] = T(0);
-      half_product(tile, y, T(1));
-#pragma unroll
-      for (int q = 0; q < NR; ++q) part[h][r][q] = (y[0][q] + y[1][q]) + (y[2][q] + y[3][q]);
-      __syncthreads();
-      if (h == 0)
-#pragma unroll
-        for (int q = 0; q < NR; ++q) d[q] = part[0][r][q] + part[1][r][q];
-      continue;
-    }
-    // the coupling: x = d - M_i x_p
-    const int ok = fill_sx(pcb);
-    if (!__syncthreads_and(ok)) {
-      cp_async_wait<0>();
-      return;
     }
     T y[4][NR];
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int q = 0; q < NR; ++q) y[j][q] = T(0);
-    half_product(tile, y, T(1));
+    if (t == nlead) {  // d = Inv_ii (right-hand side so far)
+      put_part(a);
+      __syncthreads();
+      if (h < NR) sx[r][h] = valid ? total() : T(0);
+      __syncthreads();
+      share_product(tile, y, T(1));
+      put_part(y);
+      __syncthreads();
+      if (h < NR) d = total();
+      continue;
+    }
+    // the coupling: x = d - M_i x_p
+    T m[Q];
 #pragma unroll
-    for (int q = 0; q < NR; ++q) part[h][r][q] = (y[0][q] + y[1][q]) + (y[2][q] + y[3][q]);
+    for (int c = 0; c < Q; ++c) m[c] = tile[Q * h + c][r];
+    const int ok = fill_sx(pcb);
+    if (!__syncthreads_and(ok)) break;
+#pragma unroll
+    for (int c = 0; c < Q; ++c)
+#pragma unroll
+      for (int q = 0; q < NR; ++q) y[c & 3][q] = fma(m[c], sx[Q * h + c][q], y[c & 3][q]);
+    put_part(y);
     __syncthreads();
-    if (h == 0)
-#pragma unroll
-      for (int q = 0; q < NR; ++q) d[q] -= part[0][r][q] + part[1][r][q];
+    if (h < NR) d -= total();
   }
-  cp_async_wait<0>();
-  if (h == 0 && valid)
+  cp_async_wait<0>();  // no copy may land after the CTA has left
+  if (h < nrhs && valid) {  // nrhs <= NR
+    const T v = SweepBits<T>::canon(d);
 #pragma unroll
-    for (int q = 0; q < NR; ++q)
-      if (q < nrhs) {
-        const T v = SweepBits<T>::canon(d[q]);
-        if (FWD) Y[(r0 + r) + q * ldy] = v;
-        else Out[(TRANS ? (int64_t)perm[r0 + r] : r0 + r) + q * ldo] = v;
-      }
+    for (int b = 0; b < 2; ++b)
+      if (rank + 1 + b < cs && ord + 1 + b < nblk) st_cluster(pan_mapa(pan_saddr(&s_lx[b][r][h]), rank + 1 + b), v);
+    if (FWD) Y[(r0 + r) + h * ldy] = v;
+    else Out[(TRANS ? (int64_t)perm[r0 + r] : r0 + r) + h * ldo] = v;
+  }
+  cluster_sync_all();  // a CTA stays until nothing more can be pushed to it
 }
 
 template <typename T>
@@ -686,7 +738,7 @@ void getrs_carve(GetrsPlan<T>& p, void* base, size_t bytes, int64_t work_cols) {
 
 namespace {
 template <typename T, int NR, bool TRANS, bool FWD>
-void launch_sweep(const GetrsPlan<T>& p, int nr, T* B, int64_t ldb, cudaStream_t s) {
+cudaError_t launch_sweep(const GetrsPlan<T>& p, int nr, T* B, int64_t ldb, cudaStream_t s) {
   const int64_t nblk = (p.n + kTS - 1) / kTS;
   const T* In = FWD ? B : nullptr;
   T* Out = FWD ? nullptr : B;
@@ -694,12 +746,27 @@ void launch_sweep(const GetrsPlan<T>& p, int nr, T* B, int64_t ldb, cudaStream_t
   // n^2 flops per right-hand side
   LaunchScope ls(K_SOLVE, (double)p.n * (double)p.n * nr,
                  0.5 * (double)p.n * (double)p.n * sizeof(T) + 2.0 * p.n * nr * sizeof(T), s);
-  if (p.fast && p.inv)
-    fast_sweep_kernel<T, NR, TRANS, FWD><<<(unsigned)(nblk * ((nr + NR - 1) / NR)), kSweepThreads, sweep_smem<T>(), s>>>(
-        p.n, p.LU, p.lda, p.perm, In, ldb, p.work, p.n, Out, ldb, nr, p.scratch, p.inv);
-  else
-    solve_sweep_kernel<T, TRANS, FWD><<<(unsigned)(nblk * nr), kSweepThreads, sweep_smem<T>(), s>>>(
-        p.n, p.LU, p.lda, p.perm, In, ldb, p.work, p.n, Out, ldb, nr, p.scratch);
+  if (p.fast && p.inv) {
+    // clusters of eight block rows (of fewer for fewer)
+    const int cs = nblk >= 8 ? 8 : nblk >= 4 ? 4 : nblk >= 2 ? 2 : 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((nblk + cs - 1) / cs * cs * ((nr + NR - 1) / NR)));
+    cfg.blockDim = dim3(kTS * kFastSplit<T>);
+    cfg.dynamicSmemBytes = sweep_smem<T>();
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cs;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, fast_sweep_kernel<T, NR, TRANS, FWD>, p.n, p.LU, p.lda, p.perm, In, ldb, p.work,
+                              p.n, Out, ldb, nr, p.scratch, p.inv);
+  }
+  solve_sweep_kernel<T, TRANS, FWD><<<(unsigned)(nblk * nr), kSweepThreads, sweep_smem<T>(), s>>>(
+      p.n, p.LU, p.lda, p.perm, In, ldb, p.work, p.n, Out, ldb, nr, p.scratch);
+  return cudaGetLastError();
 }
 
 template <typename T, int NR>
@@ -710,17 +777,13 @@ cudaError_t run_chunk(const GetrsPlan<T>& p, char trans, int nr, T* B, int64_t l
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(&p.scratch->ticket, 0, sizeof(unsigned), s);
   if (e != cudaSuccess) return e;
-  if (tr) launch_sweep<T, NR, true, true>(p, nr, B, ldb, s);
-  else launch_sweep<T, NR, false, true>(p, nr, B, ldb, s);
-  e = cudaGetLastError();
+  e = tr ? launch_sweep<T, NR, true, true>(p, nr, B, ldb, s) : launch_sweep<T, NR, false, true>(p, nr, B, ldb, s);
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(&p.scratch->ticket, 0, sizeof(unsigned), s);
   if (e != cudaSuccess) return e;
   e = cudaMemset2DAsync(B, ldb * sizeof(T), 0xFF, p.n * sizeof(T), nr, s);
   if (e != cudaSuccess) return e;
-  if (tr) launch_sweep<T, NR, true, false>(p, nr, B, ldb, s);
-  else launch_sweep<T, NR, false, false>(p, nr, B, ldb, s);
-  return cudaGetLastError();
+  return tr ? launch_sweep<T, NR, true, false>(p, nr, B, ldb, s) : launch_sweep<T, NR, false, false>(p, nr, B, ldb, s);
 }
 
 template <typename T, int NR>
@@ -748,8 +811,6 @@ void getrs_configure(int /*device*/) {
   configure_fast<double, 1>();
   configure_fast<float, 1>();
   configure_fast<float, 2>();
-  configure_fast<float, 4>();
-  configure_fast<float, 8>();
 }
 
 template <typename T>
@@ -762,11 +823,7 @@ cudaError_t getrs_launch(const GetrsPlan<T>& p, char trans, int64_t nrhs, T* B, 
     T* Bc = B + c * ldb;
     cudaError_t e;
     if (sizeof(T) == 8 || nr == 1) e = run_chunk<T, 1>(p, trans, nr, Bc, ldb, s);
-    else if constexpr (sizeof(T) == 4) {
-      if (nr == 2) e = run_chunk<T, 2>(p, trans, nr, Bc, ldb, s);
-      else if (nr <= 4) e = run_chunk<T, 4>(p, trans, nr, Bc, ldb, s);
-      else e = run_chunk<T, 8>(p, trans, nr, Bc, ldb, s);
-    }
+    else e = run_chunk<T, sizeof(T) == 8 ? 1 : 2>(p, trans, nr, Bc, ldb, s);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
