@@ -358,7 +358,7 @@ int32_t gblu_factor_create(gblu_ctx* ctx, int64_t m, int64_t n, int32_t precisio
     // Panel pivoting of the low-precision factors: partial pivoting (the
     // reference's order) by default; GBLU_PANEL=tournament at creation
     // selects tournament pivoting for leaves taller than 512 rows (slower
-    // on this GPU than the register cluster panel: two dependent getf2
+    // on this GPU than the sub-panel cluster kernel: two dependent getf2
     // passes per leaf against one).
     {
       const char* pe = getenv("GBLU_PANEL");

@@ -10,7 +10,7 @@
 // (trans = 'T') is U^T y = b, L^T z = y, x = P^T z as LAPACK dgetrs 'T'.
 //
 // Parallel structure: the matrix is cut into 64-row block rows.  Each CTA takes
-// one block row of one right-hand side by ticket (tickets are handed out in
+// one block row of one right-hand side (fast FP32: two) by ticket (handed out in
 // launch order, so every CTA waits only for CTAs already running), streams its
 // off-diagonal tiles in order, polling the published solution values right
 // before a tile needs them, then solves its diagonal block and publishes its

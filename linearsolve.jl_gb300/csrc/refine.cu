@@ -21,7 +21,7 @@
 
 namespace gblu {
 
-constexpr int kRowsPerCta = 256;
+constexpr int kRowsPerCta = 256;  // at most, gemv_n_partial_kernel
 constexpr int kXTile = 128;  // columns of X staged in shared memory at a time
 constexpr int kMaxW = 8;
 
@@ -261,7 +261,7 @@ gemv_n_partial_kernel(int64_t rows, int64_t cols, const double* __restrict__ A, 
   const int s = blockIdx.y;
   const int64_t cs = (cols + kSplit - 1) / kSplit;
   const int64_t j0 = s * cs, j1 = min(cols, j0 + cs);
-  const int64_t i = (int64_t)blockIdx.x * kRowsPerCta + threadIdx.x;
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   double acc[W];
 #pragma unroll
   for (int q = 0; q < W; ++q) acc[q] = 0.0;
@@ -317,63 +317,36 @@ gemv_t_partial_kernel(int64_t rows, int64_t cols, const double* __restrict__ A, 
 }
 
 // out[i,q] = beta*C[i,q] + alpha*sum_s P[s][q][i]; optional column max of |out|.
-__global__ void gemv_reduce_kernel(int64_t len, int W, int Wp, const double* __restrict__ P, double alpha,
-                                   const double* __restrict__ C, int64_t ldc, double beta,
-                                   double* __restrict__ out, int64_t ldo,
-                                   unsigned long long* __restrict__ colmax) {
-  __shared__ double red[256 / 32];
-  for (int q = 0; q < W; ++q) {
-    double mx = 0.0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < len;
-         i += (int64_t)gridDim.x * blockDim.x) {
-      double sum = 0.0;
-      for (int s = 0; s < kSplit; ++s) sum += P[((size_t)s * Wp + q) * len + i];
-      double v = alpha * sum;
-      if (beta != 0.0) v = fma(beta, C[i + q * ldc], v);
-      out[i + q * ldo] = v;
-      double av = fabs(v);
-      mx = (av > mx || isnan(av)) ? av : mx;
-    }
-    if (colmax) {
-      for (int off = 16; off; off >>= 1) {
-        double o = __shfl_down_sync(0xffffffffu, mx, off);
-        mx = (o > mx || isnan(o)) ? o : mx;
-      }
-      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double m = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = (red[w] > m || isnan(red[w])) ? red[w] : m;
-        atomic_max_nonneg(colmax + q, m);
-      }
-      __syncthreads();
-    }
+// One column per blockIdx.y.
+__global__ void __launch_bounds__(256)
+gemv_reduce_kernel(int64_t len, int Wp, const double* __restrict__ P, double alpha, const double* __restrict__ C,
+                   int64_t ldc, double beta, double* __restrict__ out, int64_t ldo,
+                   unsigned long long* __restrict__ colmax) {
+  const int q = blockIdx.y;
+  double mx = 0.0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < len; i += (int64_t)gridDim.x * blockDim.x) {
+    double sum = 0.0;
+#pragma unroll
+    for (int s = 0; s < kSplit; ++s) sum += P[((size_t)s * Wp + q) * len + i];
+    double v = alpha * sum;
+    if (beta != 0.0) v = fma(beta, C[i + q * ldc], v);
+    out[i + q * ldo] = v;
+    const double av = fabs(v);
+    mx = (av > mx || isnan(av)) ? av : mx;
   }
+  if (colmax) block_max_into(mx, colmax + q);
 }
 
-__global__ void colmax_kernel(int64_t n, int W, const double* __restrict__ X, int64_t ldx,
-                              unsigned long long* __restrict__ colmax) {
-  __shared__ double red[256 / 32];
-  for (int q = 0; q < W; ++q) {
-    double mx = 0.0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-      double av = fabs(X[i + q * ldx]);
-      mx = (av > mx || isnan(av)) ? av : mx;
-    }
-    for (int off = 16; off; off >>= 1) {
-      double o = __shfl_down_sync(0xffffffffu, mx, off);
-      mx = (o > mx || isnan(o)) ? o : mx;
-    }
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double m = 0.0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = (red[w] > m || isnan(red[w])) ? red[w] : m;
-      atomic_max_nonneg(colmax + q, m);
-    }
-    __syncthreads();
+// max |X[:,q]|, one column per blockIdx.y
+__global__ void __launch_bounds__(256)
+colmax_kernel(int64_t n, const double* __restrict__ X, int64_t ldx, unsigned long long* __restrict__ colmax) {
+  const int q = blockIdx.y;
+  double mx = 0.0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const double av = fabs(X[i + q * ldx]);
+    mx = (av > mx || isnan(av)) ? av : mx;
   }
+  block_max_into(mx, colmax + q);
 }
 
 // The power-of-two scale 2^ilogb(m) of a column from its maximum's bit pattern
@@ -676,9 +649,6 @@ size_t refine_bytes(int64_t n, int64_t W) {
   b += align256((size_t)n * W * sizeof(double));           // w
   b += align256(3 * (kGmresRestart + 1) * W * sizeof(double));  // h
   b += align256(4 * W * sizeof(unsigned long long));       // colmax
-  b += align256((size_t)kDotBlocks * (kGmresRestart + 1) * sizeof(double));
-  b += align256(4 * sizeof(double) * kMaxW);               // scales
-  b += align256(sizeof(double));                           // anorm
   b += align256(2 * sizeof(unsigned long long));           // growth words
   b += align256((size_t)W * kGmStride * sizeof(double));   // GMRES state
   b += align256((size_t)W * 2 * sizeof(int));              // GMRES flags
@@ -701,8 +671,6 @@ void refine_carve(RefineWork& w, char* base, int64_t n, int64_t W) {
   w.w = reinterpret_cast<double*>(take((size_t)n * W * sizeof(double)));
   w.h = reinterpret_cast<double*>(take(3 * (kGmresRestart + 1) * W * sizeof(double)));
   w.colmax = reinterpret_cast<unsigned long long*>(take(4 * W * sizeof(unsigned long long)));
-  w.dots = reinterpret_cast<double*>(take((size_t)kDotBlocks * (kGmresRestart + 1) * sizeof(double)));
-  w.anorm_dev = reinterpret_cast<double*>(take(4 * sizeof(double) * kMaxW));
   w.growth_bits = reinterpret_cast<unsigned long long*>(take(2 * sizeof(unsigned long long)));
   w.gm = reinterpret_cast<double*>(take((size_t)W * kGmStride * sizeof(double)));
   w.gflags = reinterpret_cast<int*>(take((size_t)W * 2 * sizeof(int)));
@@ -715,6 +683,25 @@ unsigned grid_for(int64_t n, int threads = 256) {
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>(b, 152 * 8));
 }
 
+// Rows of a CTA of gemv_n_partial_kernel.  The FP64 pipe of the busiest SM is
+// the bound, so the choice is the least ceil(CTAs / SMs) x rows, ties to the
+// larger (fewer copies of X): at n = 3000, 256 rows give 192 CTAs, two on 40 of
+// the 152 SMs, and 64 rows 752, five on the busiest (2 -> 1.25 units; the 28
+// products and corrections of a GMRES solve of four columns 13.9 -> 12.5 ms,
+// with the reduction's columns side by side).
+int gemv_rows_per_cta(int64_t rows) {
+  int device = 0;
+  cudaGetDevice(&device);
+  const int64_t sms = std::max(1, device_info(device).num_sms);
+  int best = kRowsPerCta;
+  int64_t least = 0;
+  for (int r = kRowsPerCta; r >= 64; r /= 2) {
+    const int64_t load = ((rows + r - 1) / r * kSplit + sms - 1) / sms * r;
+    if (r == kRowsPerCta || load < least) { least = load; best = r; }
+  }
+  return best;
+}
+
 // out = beta*C + alpha*op(A) X   (op(A): len x k; A stored rows x cols)
 cudaError_t gemv(char op, int64_t rows, int64_t cols, const double* A, int64_t lda, const double* X,
                  int64_t ldx, int W, double alpha, const double* C, int64_t ldc, double beta,
@@ -725,18 +712,19 @@ cudaError_t gemv(char op, int64_t rows, int64_t cols, const double* A, int64_t l
   const int Wp = W <= 1 ? 1 : W <= 2 ? 2 : W <= 4 ? 4 : 8;
   if (op == 'N') {
     len = rows;
-    dim3 grid((unsigned)((rows + kRowsPerCta - 1) / kRowsPerCta), kSplit);
+    const int cta = gemv_rows_per_cta(rows);
+    dim3 grid((unsigned)((rows + cta - 1) / cta), kSplit);
     LaunchScope ls_(K_REFINE, 2.0 * rows * cols * W, 8.0 * rows * cols, s);
     if (absval) {
-      if (Wp == 1 || X == nullptr) gemv_n_partial_kernel<1, true><<<grid, kRowsPerCta, 0, s>>>(rows, cols, A, lda, X, ldx, W, P);
-      else if (Wp == 2) gemv_n_partial_kernel<2, true><<<grid, kRowsPerCta, 0, s>>>(rows, cols, A, lda, X, ldx, W, P);
-      else if (Wp == 4) gemv_n_partial_kernel<4, true><<<grid, kRowsPerCta, 0, s>>>(rows, cols, A, lda, X, ldx, W, P);
-      else gemv_n_partial_kernel<8, true><<<grid, kRowsPerCta, 0, s>>>(rows, cols, A, lda, X, ldx, W, P);
+      if (Wp == 1 || X == nullptr) gemv_n_partial_kernel<1, true><<<grid, cta, 0, s>>>(rows, cols, A, lda, X, ldx, W, P);
+      else if (Wp == 2) gemv_n_partial_kernel<2, true><<<grid, cta, 0, s>>>(rows, cols, A, lda, X, ldx, W, P);
+      else if (Wp == 4) gemv_n_partial_kernel<4, true><<<grid, cta, 0, s>>>(rows, cols, A, lda, X, ldx, W, P);
+      else gemv_n_partial_kernel<8, true><<<grid, cta, 0, s>>>(rows, cols, A, lda, X, ldx, W, P);
     } else {
-      if (Wp == 1 || X == nullptr) gemv_n_partial_kernel<1, false><<<grid, kRowsPerCta, 0, s>>>(rows, cols, A, lda, X, ldx, W, P);
-      else if (Wp == 2) gemv_n_partial_kernel<2, false><<<grid, kRowsPerCta, 0, s>>>(rows, cols, A, lda, X, ldx, W, P);
-      else if (Wp == 4) gemv_n_partial_kernel<4, false><<<grid, kRowsPerCta, 0, s>>>(rows, cols, A, lda, X, ldx, W, P);
-      else gemv_n_partial_kernel<8, false><<<grid, kRowsPerCta, 0, s>>>(rows, cols, A, lda, X, ldx, W, P);
+      if (Wp == 1 || X == nullptr) gemv_n_partial_kernel<1, false><<<grid, cta, 0, s>>>(rows, cols, A, lda, X, ldx, W, P);
+      else if (Wp == 2) gemv_n_partial_kernel<2, false><<<grid, cta, 0, s>>>(rows, cols, A, lda, X, ldx, W, P);
+      else if (Wp == 4) gemv_n_partial_kernel<4, false><<<grid, cta, 0, s>>>(rows, cols, A, lda, X, ldx, W, P);
+      else gemv_n_partial_kernel<8, false><<<grid, cta, 0, s>>>(rows, cols, A, lda, X, ldx, W, P);
     }
   } else {
     len = cols;
@@ -751,7 +739,7 @@ cudaError_t gemv(char op, int64_t rows, int64_t cols, const double* A, int64_t l
   if (e != cudaSuccess) return e;
   { LaunchScope ls_(K_REFINE, 0.0, 0.0, s);
   const int Wp_used = (op == 'N' && X == nullptr) ? 1 : Wp;
-  gemv_reduce_kernel<<<grid_for(len), 256, 0, s>>>(len, W, Wp_used, P, alpha, C, ldc, beta, out, ldo, colmax);
+  gemv_reduce_kernel<<<dim3(grid_for(len), W), 256, 0, s>>>(len, Wp_used, P, alpha, C, ldc, beta, out, ldo, colmax);
   }
   return cudaGetLastError();
 }
@@ -942,7 +930,7 @@ struct Solver {
             "residual");
     if (!x_known) {
       LaunchScope ls_(K_REFINE, 0.0, 0.0, s);
-      colmax_kernel<<<grid_for(n), 256, 0, s>>>(n, W, w.x, n, w.colmax + w.W);
+      colmax_kernel<<<dim3(grid_for(n), W), 256, 0, s>>>(n, w.x, n, w.colmax + w.W);
     }
     GBLU_CK(ctx, cudaGetLastError(), "colmax");
     std::vector<unsigned long long> bits(2 * w.W);
@@ -962,7 +950,7 @@ struct Solver {
     GBLU_CK(ctx, cudaMemsetAsync(w.colmax, 0, w.W * sizeof(unsigned long long), s), "memset");
     GBLU_CK(ctx, cudaMemcpyAsync(w.r, w.b, (size_t)n * W * sizeof(double), cudaMemcpyDeviceToDevice, s), "r = b");
     { LaunchScope ls_(K_REFINE, 0.0, 0.0, s);
-    colmax_kernel<<<grid_for(n), 256, 0, s>>>(n, W, w.b, n, w.colmax);
+    colmax_kernel<<<dim3(grid_for(n), W), 256, 0, s>>>(n, w.b, n, w.colmax);
     }
     GBLU_CK(ctx, cudaGetLastError(), "colmax");
     std::vector<unsigned long long> bits(w.W);
@@ -1202,7 +1190,7 @@ int32_t refine_solve(gblu_ctx* ctx, gblu_factor* f, char trans, int64_t nrhs, do
         GBLU_CK(ctx, cudaMemsetAsync(w.colmax + 2 * w.W, 0, nc * sizeof(unsigned long long), s), "memset");
         {
           LaunchScope ls_(K_REFINE, 0.0, 0.0, s);
-          colmax_kernel<<<grid_for(n), 256, 0, s>>>(n, nc, w.b, n, w.colmax + 2 * w.W);
+          colmax_kernel<<<dim3(grid_for(n), nc), 256, 0, s>>>(n, w.b, n, w.colmax + 2 * w.W);
         }
         std::vector<unsigned long long> bits(nc);
         GBLU_CK(ctx, cudaMemcpyAsync(bits.data(), w.colmax + 2 * w.W, nc * sizeof(unsigned long long),

@@ -21,11 +21,9 @@ struct RefineWork {
   double* partial = nullptr;  // kSplit x n x W  deterministic partial sums
   double* V = nullptr;      // n x (restart + 1) x W   GMRES bases, one per column
   double* w = nullptr;      // n x W    GMRES work vectors
-  double* h = nullptr;      // 3 x (restart + 1) x W   projections and norms
+  double* h = nullptr;      // 3 x (restart + 1) x W   projections (two passes)
   unsigned long long* colmax = nullptr;  // 4 x W   |.|_inf per column (bit patterns)
-  double* dots = nullptr;   // kDotBlocks x (restart + 1)
   double anorm = 0;         // ||A||_inf of the FP64 matrix (host copy)
-  double* anorm_dev = nullptr;
   double amax = 0;          // max |A_ij| of the FP64 matrix (host copy)
   unsigned long long* growth_bits = nullptr;  // [0] max|A| (FP64 bits), [1] max|U| (FP32 bits)
   // GMRES state on the device, per column: Hessenberg matrix, rotations,
@@ -36,7 +34,6 @@ struct RefineWork {
 };
 
 constexpr int kSplit = 16;       // column chunks of the residual GEMV
-constexpr int kDotBlocks = 64;   // blocks of the deterministic dot products
 constexpr int kGmresRestart = 30;
 // per-column GMRES state: H ((m+1) x m), cs (m), sn (m), g (m+1), y (m+1),
 // beta, 1/norm of the newest basis vector
