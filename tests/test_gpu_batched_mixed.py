@@ -64,3 +64,39 @@ def test_fp64_resolve(ctx, pkg, oracle_mod, n, kind):
         assert np.array_equal(xs[1], oracle_mod.getrs(LU, ipiv, bs[1]), equal_nan=True)
     for i in (0, 2):
         assert oracle_mod.backward_error(As[i], xs[i], bs[i]) <= 10 * n * EPS64
+
+
+@pytest.mark.parametrize("n,count", [(80, 1500), (150, 900), (200, 500), (240, 500)])
+def test_singular_systems_leave_the_others_alone(ctx, pkg, n, count):
+    """More systems than CTAs, every third one with a zero FP32 pivot (all zero,
+    a zero column, entries below the FP32 range): the systems that follow in
+    the same CTA are refined and have the bits they have without them."""
+    rng = np.random.default_rng(n)
+    As = rng.standard_normal((count, n, n)) + 2 * np.sqrt(n) * np.eye(n)
+    bs = rng.standard_normal((count, n))
+    bad = np.arange(count) % 3 == 1
+    kind = np.arange(count) // 3 % 3
+    As[bad & (kind == 0)] = 0.0
+    As[bad & (kind == 1), n // 2, :] = 0.0  # stored by columns: a zero column
+    As[bad & (kind == 2)] *= 1e-60
+
+    def solve(sel):
+        bt = pkg.Batch(ctx, [n] * int(sel.sum()), "fp32")
+        x = bt.solve(As[sel].ravel(), bs[sel].ravel()).reshape(-1, n)
+        it, info = bt.iterations(), bt.info.copy()
+        bt.close()
+        return x, it, info
+
+    x, it, info = solve(np.ones(count, bool))
+    xg, itg, infog = solve(~bad)
+    assert (itg >= 0).all() and (infog == 0).all()
+    assert np.array_equal(it[~bad], itg)
+    assert np.array_equal(x[~bad], xg)
+    assert (it[bad] == -1).all()
+    assert (info[bad & (kind == 0)] == 1).all()
+    assert (info[bad & (kind == 1)] == n // 2 + 1).all()
+    tiny = bad & (kind == 2)
+    assert (info[tiny] == 0).all()
+    r = np.einsum("sji,sj->si", As[tiny], x[tiny]) - bs[tiny]  # row i of A is As[:, i]
+    scale = np.abs(As[tiny]).sum(1).max(1) * np.abs(x[tiny]).max(1) + np.abs(bs[tiny]).max(1)
+    assert (np.abs(r).max(1) <= 10 * n * EPS64 * scale).all()
