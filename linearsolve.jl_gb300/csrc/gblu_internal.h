@@ -124,14 +124,15 @@ void genp_configure(int device);
 cudaError_t genp_panel_launch(float* A, int64_t lda, int64_t m, int64_t c0, int w, int64_t* ipiv,
                               int64_t* info, void* work, float* linv, cudaStream_t s);
 
-// Sub-panel cluster kernel (panel.cu).  panel_sub_width: the leaf width it takes
+// Sub-panel cluster kernel (panel.cu).  panel_sub_configure: sets it up on
+// `device`, the current one.  panel_sub_width: the leaf width it takes
 // for a leaf of M rows, 0 when it does not take it (or no cluster of 16 CTAs
-// can be launched).  The launch factors columns c0 .. c0 + w - 1 of rows
+// can be launched on the device).  The launch factors columns c0 .. c0 + w - 1 of rows
 // c0 .. m - 1 and leaves the leaf's interchanges in *moves.
 template <typename T>
-bool panel_sub_ready();
+void panel_sub_configure(int device);
 template <typename T>
-int panel_sub_width(int64_t M);
+int panel_sub_width(int device, int64_t M);
 template <typename T>
 cudaError_t panel_sub_launch(T* A, int64_t lda, int64_t m, int64_t c0, int w, int64_t* ipiv, int64_t* info,
                              LeafMoves* moves, DevScratch* scr, cudaStream_t s);

@@ -1152,7 +1152,7 @@ struct Driver {
   int sub_width(int64_t c0) const {
     if (forced == 1 || forced == 2 || !p.use_sub_panel || !p.moves) return 0;
     if (std::is_same<T, float>::value && ((p.nopivot && p.tslu_work) || (p.tslu && p.tslu_work && p.m - c0 > 512))) return 0;
-    return panel_sub_width<T>(p.m - c0);
+    return panel_sub_width<T>(device, p.m - c0);
   }
   int leaf_width(int64_t c0) const {
     if (std::is_same<T, float>::value && p.nopivot && p.tslu_work) return kGenpW;
@@ -1431,8 +1431,8 @@ void getrf_configure(int device) {
   cudaFuncSetAttribute(panel_cluster_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
   cudaFuncSetAttribute(panel_cluster_kernel<double>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   cudaFuncSetAttribute(panel_cluster_kernel<float>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  panel_sub_ready<double>();
-  panel_sub_ready<float>();
+  panel_sub_configure<double>(device);
+  panel_sub_configure<float>(device);
   cudaFuncSetAttribute(trsm_lunit_kernel<double, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)trsm_smem<double, 128>());
   cudaFuncSetAttribute(trsm_lunit_kernel<float, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -3,7 +3,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <mutex>
 
 #include "gblu_internal.h"
 #include "panel.cuh"
@@ -98,23 +97,32 @@ cudaError_t sub_dispatch(int v, T* A, int64_t lda, int64_t m, int64_t c0, int w,
 
 }  // namespace
 
+namespace {
+
+// Per device, as the kernels' attributes are (cudaFuncSetAttribute changes them
+// for the current device only).
 template <typename T>
-bool panel_sub_ready() {
-  static std::once_flag once;
-  static bool ok = false;
-  std::call_once(once, [] {
-    ok = true;
-    for (int v = 1; v <= (sizeof(T) == 8 ? 5 : 6); ++v)
-      ok = ok && sub_dispatch<T>(v, nullptr, 0, 0, 0, 0, nullptr, nullptr, nullptr, nullptr, kSubMaxCtas, true,
-                                 nullptr) == cudaSuccess;
-    cudaGetLastError();
-  });
-  return ok;
+bool& sub_ready(int device) {
+  static bool ready[64] = {false};
+  return ready[device];
+}
+
+}  // namespace
+
+template <typename T>
+void panel_sub_configure(int device) {
+  if (device < 0 || device >= 64) return;
+  bool ok = true;
+  for (int v = 1; v <= (sizeof(T) == 8 ? 5 : 6); ++v)
+    ok = ok && sub_dispatch<T>(v, nullptr, 0, 0, 0, 0, nullptr, nullptr, nullptr, nullptr, kSubMaxCtas, true,
+                               nullptr) == cudaSuccess;
+  cudaGetLastError();
+  sub_ready<T>(device) = ok;
 }
 
 template <typename T>
-int panel_sub_width(int64_t M) {
-  if (sub_variant<T>(M) == 0 || !panel_sub_ready<T>()) return 0;
+int panel_sub_width(int device, int64_t M) {
+  if (device < 0 || device >= 64 || sub_variant<T>(M) == 0 || !sub_ready<T>(device)) return 0;
   if (sizeof(T) == 8) return M <= 4096 ? 64 : 32;
   return M <= 4096 ? 128 : M <= 8192 ? 64 : 32;
 }
@@ -126,10 +134,10 @@ cudaError_t panel_sub_launch(T* A, int64_t lda, int64_t m, int64_t c0, int w, in
   return sub_dispatch<T>(sub_variant<T>(M), A, lda, m, c0, w, ipiv, info, moves, scr, sub_ctas<T>(M), false, s);
 }
 
-template bool panel_sub_ready<double>();
-template bool panel_sub_ready<float>();
-template int panel_sub_width<double>(int64_t);
-template int panel_sub_width<float>(int64_t);
+template void panel_sub_configure<double>(int);
+template void panel_sub_configure<float>(int);
+template int panel_sub_width<double>(int, int64_t);
+template int panel_sub_width<float>(int, int64_t);
 template cudaError_t panel_sub_launch<double>(double*, int64_t, int64_t, int64_t, int, int64_t*, int64_t*, LeafMoves*,
                                               DevScratch*, cudaStream_t);
 template cudaError_t panel_sub_launch<float>(float*, int64_t, int64_t, int64_t, int, int64_t*, int64_t*, LeafMoves*,
