@@ -192,9 +192,7 @@ solve_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32
   T* dst = nullptr;   // where this row's solution is published
   if (valid) {
     const int64_t prow = (FWD != TRANS) ? (int64_t)perm[r0 + r] : r0 + r;
-    // NaN canonical from here on (arithmetic gives no other), so no published
-    // value is the sentinel
-    acc = SB::canon(FWD ? In[TRANS ? r0 + r : prow] : Y[r0 + r]);
+    acc = FWD ? In[TRANS ? r0 + r : prow] : Y[r0 + r];
     dst = FWD ? Y + r0 + r : Out + (TRANS ? prow : r0 + r);
   }
   const int noff = FWD ? blk : nblk - 1 - blk;  // off-diagonal tiles of this block row
@@ -323,7 +321,10 @@ solve_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32
     }
   }
   // The chain: in each step the owner's value is final, goes to every lane, is
-  // published, and updates the rows after it.  The finished rows' registers are
+  // published, and updates the rows after it.  What is published has NaN made
+  // canonical (FP64 arithmetic keeps a NaN's payload, so an all-ones one in the
+  // factors or the right-hand side could come out as the sentinel), beside the
+  // chain, which goes on with the value as it is.  The finished rows' registers are
   // updated too and not used again, so nothing is predicated.
   if constexpr (kUnit) {
 #pragma unroll
@@ -333,8 +334,9 @@ solve_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32
       if (c >= nr) continue;  // uniform
       const T x = __shfl_sync(kAll, acc, i);
       acc = fma(-a[i], x, acc);
-      store_if(lane == i, dst, x);
-      if (first) store_shared_if(lane == i, &s_dx[c], x);
+      const T v = SB::canon(x);
+      store_if(lane == i, dst, v);
+      if (first) store_shared_if(lane == i, &s_dx[c], v);
     }
   } else {
     // First divided by the diagonal entry (Markstein's division, every lane by
@@ -371,6 +373,7 @@ solve_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32
         }
       }
       const bool mine = (FWD ? lane : 31 - lane) / 4 == g && valid;
+      own = SB::canon(own);
       store_if(mine, dst, own);
       if (first) store_shared_if(mine, &s_dx[r], own);
     }

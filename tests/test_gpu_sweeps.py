@@ -68,3 +68,29 @@ def test_fast_transposed_sweeps(ctx, oracle_mod, n, nrhs):
     X = f.getrs(B, "T")
     assert oracle_mod.backward_error(A.T, X, B) <= 10 * n * EPS64
     f.close()
+
+
+@pytest.mark.parametrize("trans", ["N", "T"])
+@pytest.mark.parametrize("bits", [0xFFFFFFFFFFFFFFFF, 0x7FFFFFFFFFFFFFFF, 0xFFF4FFF4FFF4FFF4])
+@pytest.mark.parametrize("where", ["b", "diagonal", "above", "below", "last"])
+def test_exact_sweeps_nan_payloads(ctx, oracle_mod, trans, bits, where):
+    """NaN whose payload FP64 arithmetic carries along, the all-ones pattern of
+    a buffer filled with 0xFF among them: NaN comes out where the oracle has
+    it, and no sweep waits for a value that is there."""
+    n = 150
+    rng = np.random.default_rng(8)
+    A = np.asfortranarray(rng.standard_normal((n, n)) + 10 * np.eye(n))
+    B = np.asfortranarray(rng.standard_normal((n, 3)))
+    nan = np.array([bits], dtype=np.uint64)
+    if where == "b":
+        B.view(np.uint64)[40, 1] = nan[0]
+    else:
+        A.view(np.uint64)[{"diagonal": (70, 70), "above": (10, 120), "below": (120, 10), "last": (n - 1, n - 1)}[where]] = nan[0]
+    f = ctx.factor(n, n)
+    f.getrf(A)
+    LU, ipiv, _ = oracle_mod.getrf(A)
+    assert np.array_equal(f.factors(), LU, equal_nan=True)
+    X, Xo = f.getrs(B, trans), oracle_mod.getrs(LU, ipiv, B, trans)
+    assert np.isnan(Xo).any()
+    assert np.array_equal(X, Xo, equal_nan=True)
+    f.close()
