@@ -1,6 +1,8 @@
 """The shared-memory mixed batch kernel at the edges of its size classes:
 backward error, independence of the batch around a system, and systems that
 must reach the FP64 kernel."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -100,3 +102,28 @@ def test_singular_systems_leave_the_others_alone(ctx, pkg, n, count):
     r = np.einsum("sji,sj->si", As[tiny], x[tiny]) - bs[tiny]  # row i of A is As[:, i]
     scale = np.abs(As[tiny]).sum(1).max(1) * np.abs(x[tiny]).max(1) + np.abs(bs[tiny]).max(1)
     assert (np.abs(r).max(1) <= 10 * n * EPS64 * scale).all()
+
+
+def test_size_class_residency(ctx, pkg):
+    """A class whose CTAs have 256 threads or fewer is one of which an SM holds
+    several; a CTA alone on an SM has 512."""
+    pkg.Batch(ctx, [8], "fp32").close()  # the kernels are set up with the first batch
+    per_sm = ctx.lib._ZN4gblu23batch_mixed_ctas_per_smEiPi
+    threads = ctypes.c_int()
+    for n in range(1, 257):
+        ctas = per_sm(n, ctypes.byref(threads))
+        assert ctas >= (2 if threads.value <= 256 else 1), (n, threads.value, ctas)
+
+
+@pytest.mark.parametrize("n", [157, 159, 160, 161])
+def test_pair_class_edge(ctx, pkg, oracle_mod, n):
+    """The last size of which two fit an SM and the first that has one alone,
+    in one batch: the bits each system has by itself."""
+    sizes = [n, 161, n, 160] * 90
+    As, bs = _systems(sizes, n)
+    xs, it, info = _solve(ctx, pkg, As, bs)
+    assert (info == 0).all() and (it >= 0).all()
+    for i in range(4):
+        assert oracle_mod.backward_error(As[i], xs[i], bs[i]) <= 10 * sizes[i] * EPS64
+        alone, _, _ = _solve(ctx, pkg, [As[i]], [bs[i]])
+        assert np.array_equal(alone[0], xs[i])
