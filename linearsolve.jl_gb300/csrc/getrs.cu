@@ -192,7 +192,7 @@ solve_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32
   T* dst = nullptr;   // where this row's solution is published
   if (valid) {
     const int64_t prow = (FWD != TRANS) ? (int64_t)perm[r0 + r] : r0 + r;
-    acc = FWD ? In[TRANS ? r0 + r : prow] : Y[r0 + r];
+    acc = SB::canon(FWD ? In[TRANS ? r0 + r : prow] : Y[r0 + r]);
     dst = FWD ? Y + r0 + r : Out + (TRANS ? prow : r0 + r);
   }
   const int noff = FWD ? blk : nblk - 1 - blk;  // off-diagonal tiles of this block row
@@ -321,10 +321,7 @@ solve_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32
     }
   }
   // The chain: in each step the owner's value is final, goes to every lane, is
-  // published, and updates the rows after it.  What is published has NaN made
-  // canonical (FP64 arithmetic keeps a NaN's payload, so an all-ones one in the
-  // factors or the right-hand side could come out as the sentinel), beside the
-  // chain, which goes on with the value as it is.  The finished rows' registers are
+  // published, and updates the rows after it.  The finished rows' registers are
   // updated too and not used again, so nothing is predicated.
   if constexpr (kUnit) {
 #pragma unroll
@@ -334,9 +331,8 @@ solve_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32
       if (c >= nr) continue;  // uniform
       const T x = __shfl_sync(kAll, acc, i);
       acc = fma(-a[i], x, acc);
-      const T v = SB::canon(x);
-      store_if(lane == i, dst, v);
-      if (first) store_shared_if(lane == i, &s_dx[c], v);
+      store_if(lane == i, dst, x);
+      if (first) store_shared_if(lane == i, &s_dx[c], x);
     }
   } else {
     // First divided by the diagonal entry (Markstein's division, every lane by
@@ -367,13 +363,12 @@ solve_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32
         for (int st = 4 * g; st < 4 * g + 4; ++st) {
           const int i = FWD ? st : 31 - st;
           if (32 * warp + i >= nr) continue;
-          const T x = __shfl_sync(kAll, divide_ieee(acc, dg), i);
+          const T x = SB::canon(__shfl_sync(kAll, divide_ieee(acc, dg), i));
           own = lane == i ? x : own;
           acc = fma(-dt[32 * warp + i][r], x, acc);
         }
       }
       const bool mine = (FWD ? lane : 31 - lane) / 4 == g && valid;
-      own = SB::canon(own);
       store_if(mine, dst, own);
       if (first) store_shared_if(mine, &s_dx[r], own);
     }
@@ -740,6 +735,25 @@ void getrs_carve(GetrsPlan<T>& p, void* base, size_t bytes, int64_t work_cols) {
 }
 
 namespace {
+// Columns x[:, 0 .. gridDim.y - 1] filled with the sentinel, and the ticket of
+// the sweep that follows reset.  (A byte fill cannot write a signalling NaN.)
+template <typename T>
+__global__ void __launch_bounds__(256)
+sentinel_kernel(int64_t n, T* __restrict__ x, int64_t ldx, unsigned* __restrict__ ticket) {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *ticket = 0u;
+  typename SweepBits<T>::U* c = reinterpret_cast<typename SweepBits<T>::U*>(x + blockIdx.y * ldx);
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    c[i] = SweepBits<T>::kSentinel;
+}
+
+template <typename T>
+cudaError_t sentinel_launch(const GetrsPlan<T>& p, int nr, T* x, int64_t ldx, cudaStream_t s) {
+  LaunchScope ls(K_OTHER, 0.0, (double)p.n * nr * sizeof(T), s);
+  const unsigned ctas = (unsigned)std::min<int64_t>((p.n + 255) / 256, 1024);
+  sentinel_kernel<T><<<dim3(ctas, (unsigned)nr), 256, 0, s>>>(p.n, x, ldx, &p.scratch->ticket);
+  return cudaGetLastError();
+}
+
 template <typename T, int NR, bool TRANS, bool FWD>
 cudaError_t launch_sweep(const GetrsPlan<T>& p, int nr, T* B, int64_t ldb, cudaStream_t s) {
   const int64_t nblk = (p.n + kTS - 1) / kTS;
@@ -776,15 +790,11 @@ template <typename T, int NR>
 cudaError_t run_chunk(const GetrsPlan<T>& p, char trans, int nr, T* B, int64_t ldb, cudaStream_t s) {
   const bool tr = trans == 'T' || trans == 't' || trans == 'C' || trans == 'c';
   // dependents poll Y (forward) and B (backward): fill both with the sentinel
-  cudaError_t e = cudaMemsetAsync(p.work, 0xFF, (size_t)p.n * nr * sizeof(T), s);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(&p.scratch->ticket, 0, sizeof(unsigned), s);
+  cudaError_t e = sentinel_launch(p, nr, p.work, p.n, s);
   if (e != cudaSuccess) return e;
   e = tr ? launch_sweep<T, NR, true, true>(p, nr, B, ldb, s) : launch_sweep<T, NR, false, true>(p, nr, B, ldb, s);
   if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(&p.scratch->ticket, 0, sizeof(unsigned), s);
-  if (e != cudaSuccess) return e;
-  e = cudaMemset2DAsync(B, ldb * sizeof(T), 0xFF, p.n * sizeof(T), nr, s);
+  e = sentinel_launch(p, nr, B, ldb, s);
   if (e != cudaSuccess) return e;
   return tr ? launch_sweep<T, NR, true, false>(p, nr, B, ldb, s) : launch_sweep<T, NR, false, false>(p, nr, B, ldb, s);
 }

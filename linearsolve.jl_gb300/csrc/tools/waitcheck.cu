@@ -3,7 +3,7 @@
 // expected error code, leaving the context usable.
 //   which 0: the cooperative panel's grid barrier (a count nothing reaches)
 //   which 1: getrs value polling (a sentinel nothing overwrites)
-//   which 2: the register panel's mbarrier wait (a phase nothing completes)
+//   which 2: the sub-panel kernel's mbarrier wait (a phase nothing completes)
 // No trap, no fault, no endless loop: each wait reads %globaltimer and
 // returns.
 #include <cuda_runtime.h>
@@ -50,7 +50,8 @@ extern "C" int32_t gblu_tool_waitcheck(int32_t which, int32_t* code, int32_t* ga
     return 2;
   }
   cudaMemset(scr, 0, sizeof(gblu::DevScratch));
-  cudaMemset(sentinel, 0xFF, sizeof(double));  // the all-ones sentinel
+  const unsigned long long fill = gblu::SweepBits<double>::kSentinel;
+  cudaMemcpy(sentinel, &fill, sizeof(fill), cudaMemcpyHostToDevice);
   cudaMemset(ok, 0xFF, sizeof(int));
   const auto t0 = std::chrono::steady_clock::now();
   wait_check_kernel<<<1, 32>>>(which, scr, sentinel, ok);

@@ -11,23 +11,25 @@
 namespace gblu {
 
 // Published solution values are polled directly: the buffers a sweep's
-// dependents read are filled with an all-ones bit pattern (a NaN no
-// computation produces, outputs are written with canonical NaNs) before the
-// sweep, and each 4/8-byte value is single-copy atomic, so a value that is not
-// the sentinel is final.  This saves the flag round trip per tile.
+// dependents read are filled with a sentinel before the sweep, and each
+// 4/8-byte value is single-copy atomic, so a value that is not the sentinel is
+// final.  This saves the flag round trip per tile.  The sentinel is a
+// signalling NaN: arithmetic only returns quiet ones, whatever its operands
+// (FP64 keeps a NaN's payload, so an all-ones sentinel could come out of a
+// matrix filled with 0xFF), and what a sweep takes in unchanged goes through
+// canon().
 template <typename T>
 struct SweepBits;
 template <>
 struct SweepBits<double> {
   using U = unsigned long long;
-  static constexpr U kSentinel = ~0ull;
+  static constexpr U kSentinel = 0xfff4fff4fff4fff4ull;
   static __device__ __forceinline__ U load(const double* p) {
     U v;
     asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
   }
   static __device__ __forceinline__ double as_t(U v) { return __longlong_as_double((long long)v); }
-  static __device__ __forceinline__ U bits(double v) { return (U)__double_as_longlong(v); }
   // NaN -> the canonical quiet NaN, on the integer pipe
   static __device__ __forceinline__ double canon(double v) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(v);
@@ -37,14 +39,13 @@ struct SweepBits<double> {
 template <>
 struct SweepBits<float> {
   using U = unsigned;
-  static constexpr U kSentinel = ~0u;
+  static constexpr U kSentinel = 0xffa00001u;
   static __device__ __forceinline__ U load(const float* p) {
     U v;
     asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
   }
   static __device__ __forceinline__ float as_t(U v) { return __uint_as_float(v); }
-  static __device__ __forceinline__ U bits(float v) { return __float_as_uint(v); }
   static __device__ __forceinline__ float canon(float v) {
     return (__float_as_uint(v) << 1) > 0xff000000u ? __uint_as_float(0x7fc00000u) : v;
   }

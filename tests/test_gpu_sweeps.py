@@ -71,7 +71,7 @@ def test_fast_transposed_sweeps(ctx, oracle_mod, n, nrhs):
 
 
 @pytest.mark.parametrize("trans", ["N", "T"])
-@pytest.mark.parametrize("bits", [0xFFFFFFFFFFFFFFFF, 0x7FFFFFFFFFFFFFFF, 0xFFF4FFF4FFF4FFF4])
+@pytest.mark.parametrize("bits", [0xFFFFFFFFFFFFFFFF, 0x7FFFFFFFFFFFFFFF, 0xFFF4FFF4FFF4FFF4, 0xFFFCFFF4FFF4FFF4])
 @pytest.mark.parametrize("where", ["b", "diagonal", "above", "below", "last"])
 def test_exact_sweeps_nan_payloads(ctx, oracle_mod, trans, bits, where):
     """NaN whose payload FP64 arithmetic carries along, the all-ones pattern of
