@@ -174,29 +174,20 @@ __device__ __forceinline__ T div_markstein(T a, T b, T y) {
   return fma(r, y, q);
 }
 
-// a[i] / b for N > 1 dividends with one divisor, as N independent chains
-// without branches in the common case (so the compiler can interleave them;
-// with one dividend the plain div_markstein is faster).  A zero
-// dividend gives q = a*y, which is the correctly signed zero a/b; any other
-// operand outside the safe range sends all N through the IEEE division.
-template <typename T, int N>
-__device__ __forceinline__ void div_markstein_n(T (&a)[N], T b, T y) {
-  bool bad = !DivRange<T>::in_range(y);
-  T res[N];
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    const T q = a[i] * y;
-    const bool zero = !PivKey<T>::nonzero(a[i]);
-    bad |= !zero && !DivRange<T>::in_range(q);
-    const T r = fma(-b, q, a[i]);
-    res[i] = zero ? q : fma(r, y, q);
-  }
-  if (bad) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) res[i] = a[i] / b;
-  }
-#pragma unroll
-  for (int i = 0; i < N; ++i) a[i] = res[i];
+// RN(1 / x): Newton's iteration on the hardware approximation (within two
+// units in the last place).  The second step starts within one, its remainder
+// 1 - x y is exact, and its result is then the correctly rounded reciprocal
+// unless x's significand is all ones (the exception in Markstein's theorem, as
+// above); that one, and where x or 1 / x is not well inside the normal range,
+// goes to the division, out of line.
+inline __device__ __noinline__ float divide_one(float x) { return 1.0f / x; }
+__device__ __forceinline__ float recip_rn(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  y = fmaf(y, fmaf(-x, y, 1.0f), y);
+  y = fmaf(y, fmaf(-x, y, 1.0f), y);
+  const unsigned b = __float_as_uint(x);
+  return ((b >> 23) & 0xffu) - 2u < 248u && (~b & 0x7fffffu) != 0u ? y : divide_one(x);
 }
 
 // 2^127 / (2^11 m) within a few units, below 2^64, for a 53-bit significand m

@@ -111,3 +111,29 @@ extern "C" int32_t gblu_tool_recipcheck(int64_t n, uint64_t seed, uint64_t* mism
   *mism_f32 = h[1];
   return 0;
 }
+
+namespace {
+// recip_rn against 1 / x on every FP32 bit pattern (NaN results count as equal).
+__global__ void reciprncheck_kernel(unsigned long long* bad) {
+  unsigned long long b = 0;
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < 1ull << 32; i += (uint64_t)gridDim.x * blockDim.x) {
+    const float x = __uint_as_float((unsigned)i), y = gblu::recip_rn(x), r = 1.0f / x;
+    if (__float_as_uint(y) != __float_as_uint(r) && !(y != y && r != r)) ++b;
+  }
+  if (b) atomicAdd(bad, b);
+}
+}  // namespace
+
+// Counts the FP32 operands whose recip_rn differs from 1 / x.
+extern "C" int32_t gblu_tool_reciprncheck(uint64_t* mismatches) {
+  unsigned long long* d = nullptr;
+  if (cudaMalloc(&d, sizeof(unsigned long long)) != cudaSuccess) return 1;
+  cudaMemset(d, 0, sizeof(unsigned long long));
+  reciprncheck_kernel<<<152 * 8, 256>>>(d);
+  unsigned long long h = 0;
+  cudaError_t e = cudaMemcpy(&h, d, sizeof(h), cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  if (e != cudaSuccess) return 2;
+  *mismatches = h;
+  return 0;
+}

@@ -2,6 +2,7 @@
 backward error, independence of the batch around a system, and systems that
 must reach the FP64 kernel."""
 import ctypes
+import subprocess
 
 import numpy as np
 import pytest
@@ -127,3 +128,58 @@ def test_pair_class_edge(ctx, pkg, oracle_mod, n):
         assert oracle_mod.backward_error(As[i], xs[i], bs[i]) <= 10 * sizes[i] * EPS64
         alone, _, _ = _solve(ctx, pkg, [As[i]], [bs[i]])
         assert np.array_equal(alone[0], xs[i])
+
+
+RESIDUAL_C = """
+#include <math.h>
+void residual(long n, const double *a, const double *x, const double *b, double *r) {
+  for (long i = 0; i < n; ++i) {
+    double s = b[i];
+    for (long j = 0; j < n; ++j) s = fma(-a[i + j * n], x[j], s);
+    r[i] = s;
+  }
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def residual(tmp_path_factory):
+    d = tmp_path_factory.mktemp("residual")
+    (d / "r.c").write_text(RESIDUAL_C)
+    subprocess.run(["gcc", "-O2", "-shared", "-fPIC", "-o", str(d / "r.so"), str(d / "r.c"), "-lm"], check=True)
+    f = ctypes.CDLL(str(d / "r.so")).residual
+    f.argtypes = [ctypes.c_long] + 4 * [ctypes.c_void_p]
+    f.restype = None
+
+    def call(a, x, b):
+        r = np.empty_like(b)
+        f(len(b), a.ctypes.data, x.ctypes.data, b.ctypes.data, r.ctypes.data)
+        return r
+
+    return call
+
+
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -105], ids=["", "diagonal_below_range"])
+@pytest.mark.parametrize("n,count", [(3, 60), (40, 30), (64, 20), (130, 10), (200, 6), (232, 4), (233, 4), (250, 4)])
+def test_corrections_are_the_oracles(ctx, pkg, oracle_mod, residual, n, count, scale):
+    """The FP32 factors and solves behind the corrections: the oracle's FP32
+    getrf and getrs (correctly rounded reciprocals and quotients), bit for bit.
+    The condition number of 3e4 keeps the corrections from converging to the
+    same bits whatever the factors are."""
+    rng = np.random.default_rng(n)
+    As, bs = [], []
+    for _ in range(count):
+        q1, q2 = (np.linalg.qr(rng.standard_normal((n, n)))[0] for _ in range(2))
+        As.append(np.asfortranarray(q1 * np.logspace(0, -4.5, n) @ q2) * scale)
+        bs.append(rng.standard_normal(n))
+    xs, it, info = _solve(ctx, pkg, As, bs)
+    assert (info == 0).all() and (it >= 1).all(), it
+    for a, b, x, k in zip(As, bs, xs, it):
+        LU, ipiv, _ = oracle_mod.getrf(a.astype(np.float32))
+        want, r = np.zeros(n), b
+        for c in range(k):
+            if c:
+                r = residual(a, want, b)
+            s = 2.0 ** np.floor(np.log2(np.abs(r).max()))
+            want = want + s * oracle_mod.getrs(LU, ipiv, (r / s).astype(np.float32)).astype(np.float64)
+        assert np.array_equal(x, want), (np.abs(x - want).max(), k)

@@ -93,3 +93,14 @@ def test_wide_trsm_bit_exact(pkg, oracle_mod, dtype, m, extra):
     """U12 := L11 \\ A12 of a wide matrix: orders around the 32-row blocks, the
     16-byte and the element copies of L, few and many columns."""
     _check(pkg, oracle_mod, np.random.default_rng(m + extra).standard_normal((m, m + extra)).astype(dtype))
+
+
+def test_newton_reciprocal_matches_ieee():
+    """recip_rn gives 1 / x bit for bit on all 2^32 FP32 operands."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    lib = ctypes.CDLL(os.path.join(root, "linearsolve.jl_gb300", "libgblu_tools.so"))
+    lib.gblu_tool_reciprncheck.argtypes = [ctypes.POINTER(ctypes.c_uint64)]
+    lib.gblu_tool_reciprncheck.restype = ctypes.c_int32
+    m = ctypes.c_uint64()
+    assert lib.gblu_tool_reciprncheck(ctypes.byref(m)) == 0
+    assert m.value == 0, m.value
