@@ -3,20 +3,21 @@
 //
 //   1. genp_top_kernel, one CTA: LU without interchanges of the leaf's top
 //      128 x 128 block in shared memory, 32 columns at a time; it leaves the
-//      packed factors and the inverses of U's four 32 x 32 diagonal blocks in
-//      the work area.
+//      packed factors and the reciprocals of U's diagonal in the work area.
 //   2. genp_below_kernel: every 32 rows below the block solve l U = a by
-//      blocks (product with the columns before, then with a diagonal block's
-//      inverse); sixteen more CTAs compute the inverse of L11, which the TRSMs
+//      blocks (product with the columns before, then substitution in the
+//      diagonal block); sixteen more CTAs compute the inverse of L11, which the TRSMs
 //      to the right of the leaf apply.
 //
 // What bounds a factorization of a few thousand columns is the chain of dependent
 // launches, not the work in them.  A 32-column leaf (13 us, with every CTA
 // repeating the top block's factorization) needs four panels, three TRSMs and
 // three updates where this needs two launches: FP16 factor and refined solve of
-// n = 6002, two right-hand sides, 9.57 -> 6.86 ms.  The factors' residual is
-// that of substitution throughout (FP32 operands, n = 60 .. 1500: 3.6e-7 ..
-// 2.7e-6 of max |A|, both ways), the blocks inverted being 32 columns wide.
+// n = 6002, two right-hand sides, 9.57 -> 6.86 ms.  Both kernels are substitution
+// with correctly rounded reciprocals: without pivoting nothing bounds the
+// condition of U's diagonal blocks, and a product with the inverse of one leaves
+// an error of its condition times u in the rows below (8 w u |L||U| exceeded 400
+// times where the condition is 1.6^31).
 //
 // An exactly zero pivot sets info and leaves its column unscaled, as getf2.
 #include <cuda_runtime.h>
@@ -41,9 +42,8 @@ constexpr int kInvColsPerCta = kGenpThreads / 32;
 constexpr int kInvCtas = kGenpW / kInvColsPerCta;
 constexpr int kXLd = kGenpRows + 4;
 
-// Work area: the factored top block (ld 128), then U's diagonal inverses
-// [block][column][32].
-constexpr size_t kGenpWork = (size_t)(kGenpW * kGenpW + kGenpW * kB) * sizeof(float);
+// Work area: the factored top block (ld 128), then the reciprocals of U's diagonal.
+constexpr size_t kGenpWork = (size_t)(kGenpW * kGenpW + kGenpW) * sizeof(float);
 
 __device__ __forceinline__ float part_of(const float4& v, int i) {
   return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w;
@@ -54,22 +54,6 @@ __device__ __forceinline__ void st4(float* p, const float4& v) { *reinterpret_ca
 __device__ __forceinline__ void copy16(float* dst, const float* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-}
-
-__device__ __forceinline__ void bar_sync(int id, int threads) {
-  asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-__device__ __forceinline__ void bar_arrive(int id, int threads) {
-  asm volatile("barrier.cta.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
-// 1 / x: the hardware approximation and a Newton step, without the library
-// division's branch (the step is left out where it would meet an infinity).
-__device__ __forceinline__ float recip_newton(float x) {
-  float y;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  const float e = fmaf(-x, y, 1.0f);
-  return fabsf(e) < 0.5f ? fmaf(y, e, y) : y;
 }
 
 // C(32 rows at r0, 8 columns at c0) -= L(:, k .. k + 31) U(k .. k + 31, :) by one
@@ -103,38 +87,13 @@ __device__ __forceinline__ void update_tile(float* S, int r0, int c0, int k) {
   for (int jj = 0; jj < 2; ++jj) st4(c + 4 * jj * kGenpLd + r0, acc[jj]);
 }
 
-// Column `lane` of the inverse of the upper triangle of the 32 x 32 block at
-// (o, o), rd its diagonal's reciprocals, to out[column * 32 + row].
-__device__ __forceinline__ void invert_u(const float* S, int o, const float* rd, float* out) {
-  const int lane = threadIdx.x & 31;
-  float x[kB];
-#pragma unroll
-  for (int i = 0; i < kB; ++i) x[i] = i == lane ? 1.f : 0.f;
-#pragma unroll
-  for (int kr = 0; kr < kB; ++kr) {
-    const int k = kB - 1 - kr;
-    x[k] *= rd[k];
-#pragma unroll
-    for (int i4 = 0; i4 < kB / 4; ++i4) {
-      if (4 * i4 >= k) continue;
-      const float4 u = ld4(S + (o + k) * kGenpLd + o + 4 * i4);
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (4 * i4 + q < k) x[4 * i4 + q] = fmaf(-part_of(u, q), x[k], x[4 * i4 + q]);
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < kB; i += 4) st4(out + lane * kB + i, make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]));
-}
-
 // Bound by the column chain (a broadcast, a reciprocal and an update a column),
 // so everything else runs beside it.  Per 32 columns: warps 0-3 update the
 // diagonal block with the 32 columns before; warp 0 then factors it in
 // registers (lane = row) and publishes it eight columns at a time to warps 1-3
 // (a row below it a thread, l U = a) and 4-6 (a column right of it a thread,
 // L u = a), which follow eight columns behind, after the rows and columns they
-// solve have had their update; warps 7-14 update the rest and warp 15 inverts
-// the previous diagonal block's U.  Against the same steps one after the other:
+// solve have had their update; warps 7-15 update the rest.  Against the same steps one after the other:
 // 52,000 -> 45,000 cycles a 128 x 128 block.  Columns and rows past w are those
 // of the identity.
 __global__ void __launch_bounds__(kGenpTopThreads)
@@ -142,10 +101,10 @@ genp_top_kernel(float* __restrict__ A, int64_t lda, int64_t c0, int w, int64_t* 
                 int64_t* __restrict__ info, float* __restrict__ work) {
   extern __shared__ __align__(16) float S[];  // S[c * kGenpLd + r]
   __shared__ __align__(16) float UT[kB][kB + 4];  // the current diagonal block by rows
-  __shared__ float rd[2][kB];                     // reciprocals of its pivots, by block parity
+  __shared__ float rd[kB];                        // reciprocals of its pivots
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nb = (w + kB - 1) / kB, end = kB * nb;
-  float* uinv = work + kGenpW * kGenpW;
+  float* rdiag = work + kGenpW * kGenpW;
   float* Ac = A + c0 + c0 * lda;
 #pragma unroll 16
   for (int e = 0; e < kGenpW * kGenpW / kGenpTopThreads; ++e) {
@@ -161,24 +120,23 @@ genp_top_kernel(float* __restrict__ A, int64_t lda, int64_t c0, int w, int64_t* 
     if (b > 0) {
       if (warp < 4) {
         update_tile(S, o, o + 8 * warp, kp);
-        bar_sync(5, 128);
+        named_bar_sync(5, 128);
       }
       if (warp > 0) {
         for (int q = warp - 1; q < 8 * nrem; q += 15) {
           if (q < 4 * nrem) update_tile(S, o + kB + kB * (q / 4), o + 8 * (q % 4), kp);
           else update_tile(S, o, o + kB + 8 * (q - 4 * nrem), kp);
         }
-        bar_sync(6, kGenpTopThreads - 32);
+        named_bar_sync(6, kGenpTopThreads - 32);
       }
     }
-    float* rdb = rd[b & 1];
     if (warp == 0) {
       float r[kB];
 #pragma unroll
       for (int j = 0; j < kB; ++j) r[j] = S[(o + j) * kGenpLd + o + lane];
       float own = 1.f;
       float u = __shfl_sync(0xffffffffu, r[0], 0);
-      float rp = u != 0.f ? recip_newton(u) : 1.0f;
+      float rp = u != 0.f ? recip_rn(u) : 1.0f;
 #pragma unroll
       for (int k = 0; k < kB; ++k) {
         zc = (u == 0.f && zc < 0) ? o + k : zc;
@@ -191,7 +149,7 @@ genp_top_kernel(float* __restrict__ A, int64_t lda, int64_t c0, int w, int64_t* 
           const float un = __shfl_sync(0xffffffffu, r[k + 1 < kB ? k + 1 : 0], k);
           if (below) r[k + 1 < kB ? k + 1 : 0] = fmaf(-l, un, r[k + 1 < kB ? k + 1 : 0]);
           u = __shfl_sync(0xffffffffu, r[k + 1 < kB ? k + 1 : 0], k + 1);
-          rp = u != 0.f ? recip_newton(u) : 1.0f;
+          rp = u != 0.f ? recip_rn(u) : 1.0f;
         }
 #pragma unroll
         for (int j = 0; j < kB; ++j) {
@@ -204,12 +162,13 @@ genp_top_kernel(float* __restrict__ A, int64_t lda, int64_t c0, int w, int64_t* 
           for (int j = 0; j < kB; ++j)
             if (j / 8 == k / 8) S[(o + j) * kGenpLd + o + lane] = r[j];
           if (lane / 8 == k / 8) {
-            rdb[lane] = own;
+            rd[lane] = own;
+            rdiag[o + lane] = own;
 #pragma unroll
             for (int j = 0; j < kB; j += 4)
               if (j / 8 >= k / 8) st4(&UT[lane][j], make_float4(r[j], r[j + 1], r[j + 2], r[j + 3]));
           }
-          bar_arrive(1 + k / 8, 7 * 32);
+          named_bar_arrive(1 + k / 8, 7 * 32);
         }
       }
     } else if (warp < 4) {  // row t: x U_bb = a
@@ -222,9 +181,9 @@ genp_top_kernel(float* __restrict__ A, int64_t lda, int64_t c0, int w, int64_t* 
       }
 #pragma unroll
       for (int i = 0; i < kB; ++i) {
-        if ((i & 7) == 0) bar_sync(1 + i / 8, 7 * 32);
+        if ((i & 7) == 0) named_bar_sync(1 + i / 8, 7 * 32);
         if (!on) continue;
-        x[i] *= rdb[i];
+        x[i] *= rd[i];
 #pragma unroll
         for (int j4 = 0; j4 < kB / 4; ++j4) {
           if (4 * j4 + 3 <= i) continue;
@@ -251,7 +210,7 @@ genp_top_kernel(float* __restrict__ A, int64_t lda, int64_t c0, int w, int64_t* 
       }
 #pragma unroll
       for (int k = 0; k < kB; ++k) {
-        if ((k & 7) == 0) bar_sync(1 + k / 8, 7 * 32);
+        if ((k & 7) == 0) named_bar_sync(1 + k / 8, 7 * 32);
         if (!on) continue;
 #pragma unroll
         for (int i4 = 0; i4 < kB / 4; ++i4) {
@@ -267,16 +226,11 @@ genp_top_kernel(float* __restrict__ A, int64_t lda, int64_t c0, int w, int64_t* 
         for (int j = 0; j < kB; j += 4) st4(&S[t * kGenpLd + o + j], make_float4(x[j], x[j + 1], x[j + 2], x[j + 3]));
       }
     } else if (b > 0) {
-      if (warp < 15) {
-        for (int q = warp - 7; q < 4 * nrem * nrem; q += 8)
-          update_tile(S, o + kB + kB * (q % nrem), o + kB + 8 * (q / nrem), kp);
-      } else {
-        invert_u(S, kp, rd[(b - 1) & 1], uinv + (b - 1) * kB * kB);
-      }
+      for (int q = warp - 7; q < 4 * nrem * nrem; q += 9)
+        update_tile(S, o + kB + kB * (q % nrem), o + kB + 8 * (q / nrem), kp);
     }
     __syncthreads();
   }
-  if (warp == 15) invert_u(S, end - kB, rd[(nb - 1) & 1], uinv + (nb - 1) * kB * kB);
 #pragma unroll 8
   for (int e = 0; e < kGenpW * kGenpW / kGenpTopThreads; ++e) {
     const int idx = e * kGenpTopThreads + tid, c = idx / kGenpW, r = idx % kGenpW;
@@ -291,20 +245,21 @@ genp_top_kernel(float* __restrict__ A, int64_t lda, int64_t c0, int w, int64_t* 
 
 constexpr size_t kGenpTopSmem = (size_t)kGenpW * kGenpLd * sizeof(float);
 constexpr size_t kGenpBelowSmem =
-    ((size_t)kGenpW * kGenpLd + kGenpW * (kB + 4) + (size_t)kGenpW * kXLd) * sizeof(float);
+    ((size_t)kGenpW * kGenpLd + kGenpW + (size_t)kGenpW * kXLd) * sizeof(float);
 
 // CTAs 0 .. row_ctas - 1: 32 rows below the block each.  Warp: 4 rows, lane: a
 // column of the current 32, so after the copies no warp waits for another.
-// 32 rows a CTA put a 6000-row leaf on all SMs; the chain of one warp (80
-// steps of five 16-byte loads and 16 FMAs) is then what it takes.
+// 32 rows a CTA put a 6000-row leaf on all SMs; the chain of one warp (48
+// steps of five 16-byte loads and 16 FMAs, and 128 of a product, a shuffle and
+// an FMA for each of the four rows) is then what it takes.
 // The other CTAs: the inverse of L11 by the TRSM chain, one column a warp.
 __global__ void __launch_bounds__(kGenpThreads)
 genp_below_kernel(float* __restrict__ A, int64_t lda, int64_t m, int64_t c0, int w, const float* __restrict__ work,
                   int row_ctas, float* __restrict__ linv) {
   extern __shared__ __align__(16) float smem[];
   float* sU = smem;                              // the top block, by columns
-  float* sInv = sU + kGenpW * kGenpLd;           // sInv[column * 36 + k]
-  float* sX = sInv + kGenpW * (kB + 4);          // sX[column * 36 + row]
+  float* sR = sU + kGenpW * kGenpLd;             // reciprocals of U's diagonal
+  float* sX = sR + kGenpW;                       // sX[column * 36 + row]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if ((int)blockIdx.x >= row_ctas) {
     const int j0 = ((int)blockIdx.x - row_ctas) * kInvColsPerCta;
@@ -338,13 +293,12 @@ genp_below_kernel(float* __restrict__ A, int64_t lda, int64_t m, int64_t c0, int
   const int nb = (w + kB - 1) / kB;
   const int64_t r0 = c0 + w + (int64_t)blockIdx.x * kGenpRows;
   const int nr = (int)min((int64_t)kGenpRows, m - r0);
-  for (int b = 1; b < nb; ++b)  // U's blocks above the diagonal ones
-    for (int i = tid; i < kB * 8 * b; i += kGenpThreads) {
-      const int c = kB * b + i / (8 * b), k = 4 * (i % (8 * b));
+  for (int b = 0; b < nb; ++b)  // U's blocks, the diagonal ones included
+    for (int i = tid; i < kB * 8 * (b + 1); i += kGenpThreads) {
+      const int c = kB * b + i / (8 * (b + 1)), k = 4 * (i % (8 * (b + 1)));
       copy16(sU + c * kGenpLd + k, work + c * kGenpW + k);
     }
-  for (int i = tid; i < nb * kB * 8; i += kGenpThreads)
-    copy16(sInv + (i / 8) * (kB + 4) + 4 * (i % 8), work + kGenpW * kGenpW + 4 * i);
+  for (int i = tid; i < nb * kB / 4; i += kGenpThreads) copy16(sR + 4 * i, work + kGenpW * kGenpW + 4 * i);
   {
     float x[kGenpW / 8];
 #pragma unroll
@@ -376,25 +330,26 @@ genp_below_kernel(float* __restrict__ A, int64_t lda, int64_t m, int64_t c0, int
         acc.w = fmaf(-x.w, uk, acc.w);
       }
     }
-    st4(xr + c * kXLd, acc);
-    __syncwarp();
-    acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float* v = sInv + c * (kB + 4);
+    // substitution: step k's value goes from lane k to the columns after it
+    const float r = sR[c];
+    float ud[kB];
 #pragma unroll
     for (int k = 0; k < kB; k += 4) {
-      const float4 u4 = ld4(v + k);
+      const float4 u4 = ld4(u + kB * b + k);
+      ud[k] = u4.x; ud[k + 1] = u4.y; ud[k + 2] = u4.z; ud[k + 3] = u4.w;
+    }
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) {
-        const float4 x = ld4(xr + (kB * b + k + kk) * kXLd);
-        const float uk = part_of(u4, kk);
-        acc.x = fmaf(x.x, uk, acc.x);
-        acc.y = fmaf(x.y, uk, acc.y);
-        acc.z = fmaf(x.z, uk, acc.z);
-        acc.w = fmaf(x.w, uk, acc.w);
+    for (int k = 0; k < kB - 1; ++k) {
+      const float x0 = __shfl_sync(0xffffffffu, acc.x * r, k), x1 = __shfl_sync(0xffffffffu, acc.y * r, k);
+      const float x2 = __shfl_sync(0xffffffffu, acc.z * r, k), x3 = __shfl_sync(0xffffffffu, acc.w * r, k);
+      if (lane > k) {
+        acc.x = fmaf(-x0, ud[k], acc.x);
+        acc.y = fmaf(-x1, ud[k], acc.y);
+        acc.z = fmaf(-x2, ud[k], acc.z);
+        acc.w = fmaf(-x3, ud[k], acc.w);
       }
     }
-    __syncwarp();
-    st4(xr + c * kXLd, acc);
+    st4(xr + c * kXLd, make_float4(acc.x * r, acc.y * r, acc.z * r, acc.w * r));
     __syncwarp();
   }
   __syncthreads();
