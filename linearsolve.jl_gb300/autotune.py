@@ -96,7 +96,9 @@ def _time_solve(ctx, handle, dA, dB0, dB, reps: int = 2) -> float:
 def tune(ctx, sizes, precision: str = "fp32", A=None, b=None, use_cache: bool = True,
          budget_s: float = 60.0, sm_count: int | None = None) -> dict:
     """Search bucket edges x (threads, panel) per bucket x CTAs per bucket by
-    coordinate descent on the measured solve time; returns the schedule."""
+    coordinate descent on the measured solve time; returns the schedule.  FP32
+    batches take threads and panel width from each system's size (the schedule's
+    are those of the FP64 re-solve), so only edges and CTAs are searched."""
     sizes = np.ascontiguousarray(sizes, dtype=np.int64)
     sig = signature(sizes, precision)
     cache = _load_cache() if use_cache else {}
@@ -118,6 +120,7 @@ def tune(ctx, sizes, precision: str = "fp32", A=None, b=None, use_cache: bool = 
         sm_count = 152
     t_start = time.perf_counter()
     trials = []
+    variants = VARIANTS if precision == "fp64" else []
 
     def measure(s):
         apply(ctx, h, s)
@@ -136,7 +139,7 @@ def tune(ctx, sizes, precision: str = "fp32", A=None, b=None, use_cache: bool = 
                 cur["threads"][i], cur["panel"][i] = 128, 8
         ms = measure(cur)
         for i in range(nb):  # coordinate descent over each bucket's variant and CTA count
-            for (t, p) in VARIANTS:
+            for (t, p) in variants:
                 if (t, p) == (cur["threads"][i], cur["panel"][i]):
                     continue
                 cand = json.loads(json.dumps(cur))

@@ -48,3 +48,44 @@ def test_unreadable_cache_is_empty(pkg, tmp_path, monkeypatch):
     assert at._load_cache() == {}
     monkeypatch.setenv("GBLU_AUTOTUNE_FILE", str(tmp_path / "missing" / "tune.json"))
     assert at._load_cache() == {}
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_search_tries_what_has_an_effect(pkg, monkeypatch, precision):
+    """The (threads, panel) variants are timed for FP64 batches only: the mixed
+    kernel does not take them from the schedule."""
+    at = import_module(pkg.__name__ + ".autotune")
+
+    class Buffer:
+        rows = 1
+
+        def __init__(self, *a):
+            pass
+
+        @classmethod
+        def from_host(cls, x):
+            return cls()
+
+        def free(self):
+            pass
+
+    class Lib:
+        def gblu_batch_create(self, *a):
+            return 0
+
+        def gblu_batch_destroy(self, *a):
+            return 0
+
+    class Ctx:
+        lib, handle = Lib(), None
+
+    seen = []
+    monkeypatch.setattr(at, "DeviceMatrix", Buffer)
+    monkeypatch.setattr(at, "apply", lambda ctx, h, s: seen.append(s))
+    monkeypatch.setattr(at, "_time_solve", lambda *a: 1.0 + 1.0 / len(seen))  # every trial looks faster
+    best = at.tune(Ctx(), np.arange(8, 257), precision=precision, use_cache=False)
+    assert best["trials"] == len(seen)
+    starts = [s for s in seen if not any(s["ctas"])]
+    tried = {tuple(zip(s["threads"], s["panel"])) for s in seen if len(s["upper"]) == 1}
+    assert tried == ({((t, p),) for t, p in at.VARIANTS} if precision == "fp64" else {((256, 16),)})
+    assert {len(s["upper"]) for s in starts} == {len(e) for e in at.EDGE_SETS}
