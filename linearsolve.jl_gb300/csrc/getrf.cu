@@ -430,7 +430,7 @@ laswp_moves_kernel(T* __restrict__ A, int64_t lda, int64_t ncols_total, int64_t 
                    const LeafMoves* __restrict__ mv, int32_t* __restrict__ perm) {
   constexpr int MPL = 2 * kLeafMaxW / 32;  // moves per lane, at most
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nmv = mv->count;
+  const int nmv = min(mv->count, 2 * kLeafMaxW);  // no more, unless the panel gave up
   if (nmv == 0) return;
   int dst[MPL], src[MPL];
 #pragma unroll

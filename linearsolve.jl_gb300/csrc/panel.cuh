@@ -15,6 +15,7 @@ namespace gblu {
 
 constexpr int kSubW = 8;          // columns of a sub-panel
 constexpr int kSubMaxCtas = 16;
+constexpr unsigned long long kPushLandNs = 100000;  // a push takes about a microsecond
 
 // The value whose bit pattern is the key (|a| for a key of a)
 template <typename T>
@@ -221,7 +222,8 @@ panel_sub_kernel(T* __restrict__ A, int64_t lda, int64_t m, int64_t c0, int w, i
   T* Ab = A + c0 + c0 * lda;                       // the leaf's first element
   const uint32_t rx_bytes = (uint32_t)(G * 16 * PW + 16 * RB);
   int* const err = &scr->error;
-  bool bad = false;  // a wait gave up: stop waiting, finish without hanging
+  // set once a wait gave up: stop waiting, finish without hanging
+  int me = threadIdx.x;  // -1 then
   auto owner = [&](int row) { return (int)__umulhi((unsigned)row, rmagic); };  // row / R
 
   // the leaf into the tile: units of 32 rows x one 16-byte word of columns
@@ -369,10 +371,10 @@ panel_sub_kernel(T* __restrict__ A, int64_t lda, int64_t m, int64_t c0, int w, i
             if (j > 0) compose(j - 1);  // while the candidates travel
           }
           // 3. the winner over the CTAs
-          if (!bad && !pan_bar_wait(pan_saddr(&r_bar[b]), (uint32_t)(k >> 1) & 1u, err)) bad = true;
+          if (me >= 0 && !pan_bar_wait(pan_saddr(&r_bar[b]), (uint32_t)(k >> 1) & 1u, err)) me = -1;
           choose(r_pkt[b][0], pc < G ? pc : 0);
           drow = r_diag[b];
-          if (tid == 0 && k + 2 < w) pan_bar_arm(pan_saddr(&r_bar[b]), rx_bytes);  // column k + 2
+          if (me == 0 && k + 2 < w) pan_bar_arm(pan_saddr(&r_bar[b]), rx_bytes);  // column k + 2
         } else if (j > 0 && warp == 0) {
           compose(j - 1);
         }
@@ -435,11 +437,12 @@ panel_sub_kernel(T* __restrict__ A, int64_t lda, int64_t m, int64_t c0, int w, i
       if (warp == 0) {
         compose(kb - 1);  // the last column's interchange
         if (lane < NMV) {
-          s_mrow[lane] = mrow;
-          s_mfrom[lane] = mfrom;
+          // rows of the leaf, also where a wait gave up and a packet was none
+          s_mrow[lane] = min(mrow, M - 1);
+          s_mfrom[lane] = min(mfrom, M - 1);
         }
       }
-      if (warp == NWC - 1 && cta == 0 && lane < kb) ipiv[c0 + s0 + lane] = c0 + piv_row + 1;
+      if (warp == NWC - 1 && cta == 0 && lane < kb) ipiv[c0 + s0 + lane] = c0 + min(piv_row, M - 1) + 1;
     }
     __syncthreads();  // the sub-panel, its moves and the helpers' updates are in shared memory
     // 5. the interchanges on the leaf's other columns, a 16-byte word a thread.
@@ -460,7 +463,7 @@ panel_sub_kernel(T* __restrict__ A, int64_t lda, int64_t m, int64_t c0, int w, i
         if (row >= lo && row < lo + nloc && row != s_mfrom[lane]) words = 1 + nleftw + (lane < NB ? 0 : nrw);
       }
       words = __reduce_add_sync(kAll, words) + NB * nrw;
-      if (lane == 0) pan_bar_arm(pan_saddr(&r_bar[2]), 16u * (uint32_t)words);
+      if (me == 0) pan_bar_arm(pan_saddr(&r_bar[2]), 16u * (uint32_t)words);
     }
     if (nrw > 0) {
       const int e = (tid >> 4) & (NB - 1), src = s_mfrom[e];
@@ -491,7 +494,7 @@ panel_sub_kernel(T* __restrict__ A, int64_t lda, int64_t m, int64_t c0, int w, i
       }
     }
     if (G == 1) __syncthreads();
-    else if (!bad && !pan_bar_wait(pan_saddr(&r_bar[2]), (uint32_t)(s0 / NB) & 1u, err)) bad = true;
+    else if (me >= 0 && !pan_bar_wait(pan_saddr(&r_bar[2]), (uint32_t)(s0 / NB) & 1u, err)) me = -1;
     // U12 := L11 \ A12.  FP32: a thread a column; FP64: eight lanes a column
     // (a warp's FP64 instructions issue 68 cycles apart, so 28 of them in one
     // warp cost more than seven with a shuffle each)
@@ -588,6 +591,8 @@ panel_sub_kernel(T* __restrict__ A, int64_t lda, int64_t m, int64_t c0, int w, i
     if (NW > NWC && warp >= NWC) update(cn, w, NWC, NW - NWC);
   }
   __syncthreads();
+  int failed = me < 0;
+  if (G > 1 && tid == 0) failed |= ld_volatile_i32(err);  // used below, behind the stores
 #pragma unroll 4
   for (int t = warp; t < nrg * nwd; t += NW) {
     const int wd = t / nrg, i = (t - wd * nrg) * 32 + lane;
@@ -604,9 +609,23 @@ panel_sub_kernel(T* __restrict__ A, int64_t lda, int64_t m, int64_t c0, int w, i
   // the leaf's interchanges as row moves, for the other columns of the matrix
   for (int i = tid; i < nloc; i += NT) {
     const int id = *reinterpret_cast<const int*>(tile + i * LD + W);
-    if (id != lo + i) moves->mv[atomicAdd(&moves->count, 1)] = make_int2((int)c0 + lo + i, (int)c0 + id);
+    if (id != lo + i && (unsigned)id < (unsigned)M) {  // always a row, unless a wait gave up
+      const int at = atomicAdd(&moves->count, 1);
+      if (at < 2 * kLeafMaxW) moves->mv[at] = make_int2((int)c0 + lo + i, (int)c0 + id);
+    }
   }
   if (cta == 0 && tid == 0 && info_local != 0 && *info_out == 0) *info_out = info_local;
+  // No CTA leaves while another may still push to it.  Every push was waited for
+  // unless a wait gave up somewhere: then a CTA stays until the others have left
+  // or are here too, and until their last pushes have landed.
+  if (G > 1 && __syncthreads_or(failed)) {
+    cluster_arrive();
+    cluster_wait();
+    if (tid == 0) {
+      const unsigned long long t0 = global_ns();
+      while (global_ns() - t0 < kPushLandNs) {}
+    }
+  }
 }
 
 }  // namespace gblu

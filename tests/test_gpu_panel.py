@@ -104,3 +104,41 @@ def test_newton_reciprocal_matches_ieee():
     m = ctypes.c_uint64()
     assert lib.gblu_tool_reciprncheck(ctypes.byref(m)) == 0
     assert m.value == 0, m.value
+
+
+def _panelcheck(A, at):
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    f = ctypes.CDLL(os.path.join(root, "linearsolve.jl_gb300", "libgblu_tools.so")).gblu_tool_panelcheck
+    f.argtypes = [ctypes.c_int32, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int32] + 4 * [ctypes.c_void_p]
+    f.restype = ctypes.c_int32
+    A = np.array(A, order="F", copy=True)
+    ipiv, moves = np.zeros(A.shape[1], dtype=np.int64), np.zeros((256, 2), dtype=np.int32)
+    count, code = np.zeros(1, dtype=np.int32), np.zeros(1, dtype=np.int32)
+    assert f(A.dtype == np.float64, A.shape[0], A.ctypes.data, at, ipiv.ctypes.data, moves.ctypes.data,
+             count.ctypes.data, code.ctypes.data) == 0
+    return A, ipiv, moves[: min(count[0], 256)], int(code[0])
+
+
+@pytest.mark.parametrize("dtype,m", [(np.float64, 100), (np.float64, 512), (np.float32, 700)])
+@pytest.mark.parametrize("at", [-1, 0, 40, 390, 775, 1000, 2600])
+def test_late_push_gives_up_in_bounds(ctx, oracle_mod, dtype, m, at):
+    """One CTA late with one of its pushes (a candidate or a moved row) by more
+    than the wait limit: the launch ends with the error code, pivots and moves
+    name rows of the leaf, and the context goes on.  Never late: the oracle's
+    pivots and factors, and no code."""
+    A = np.random.default_rng(m).standard_normal((m, 64 if dtype == np.float64 else 128)).astype(dtype)
+    LU, ipiv, moves, code = _panelcheck(A, at)
+    assert ((ipiv >= 1) & (ipiv <= m)).all()
+    assert ((moves >= 0) & (moves < m)).all()
+    if at < 0:
+        LUo, ipivo, _ = oracle_mod.getrf(A)
+        assert code == 0
+        assert np.array_equal(ipiv, ipivo) and np.array_equal(LU, LUo)
+    else:
+        assert code == 1  # DEV_TIMEOUT_PANEL
+    B = np.random.default_rng(0).standard_normal((300, 300))
+    f = ctx.factor(300, 300)
+    assert f.getrf(B) == 0
+    assert np.array_equal(f.factors(), oracle_mod.getrf(B)[0])
+    f.close()
+
