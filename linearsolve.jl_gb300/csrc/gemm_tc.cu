@@ -433,7 +433,7 @@ bool make_map(CUtensorMap* m, const void* base, uint64_t inner, uint64_t outer, 
 
 size_t tc_work_bytes(int64_t M, int64_t N, int64_t K) {
   const int64_t Kp = ((K + 7) / 8) * 8;
-  return (size_t)(M * Kp + N * Kp) * 2 + 2 * (size_t)N * sizeof(float) + 1024;
+  return (size_t)(M * Kp + N * Kp) * 2 + (size_t)N * sizeof(float) + 1024;
 }
 
 void tc_configure(int /*device*/) {

@@ -365,7 +365,7 @@ __device__ __forceinline__ void pow2_scale(unsigned long long bits, double& scal
 }
 
 // D[:,q] = float(R[:,q] / scale_q), scale_q from the column maximum colmax[q]
-__global__ void scale_to_f32_kernel(int64_t n, int W, const double* __restrict__ R, int64_t ldr,
+__global__ void scale_to_f32_kernel(int64_t n, const double* __restrict__ R, int64_t ldr,
                                     const unsigned long long* __restrict__ colmax, float* __restrict__ D,
                                     int64_t ldd) {
   const int q = blockIdx.y;
@@ -376,7 +376,7 @@ __global__ void scale_to_f32_kernel(int64_t n, int W, const double* __restrict__
 }
 
 // X[:,q] = scale_q * double(D[:,q])
-__global__ void update_from_f32_kernel(int64_t n, int W, double* __restrict__ X, int64_t ldx,
+__global__ void update_from_f32_kernel(int64_t n, double* __restrict__ X, int64_t ldx,
                                        const float* __restrict__ D, int64_t ldd,
                                        const unsigned long long* __restrict__ colmax) {
   const int q = blockIdx.y;
@@ -882,7 +882,7 @@ struct Solver {
   int32_t precond_f32(const double* v, int64_t ldv, int W, const unsigned long long* cm) {
     {
       LaunchScope ls_(K_REFINE, 0.0, 0.0, s);
-      scale_to_f32_kernel<<<dim3(grid_for(n), W), 256, 0, s>>>(n, W, v, ldv, cm, w.d32, n);
+      scale_to_f32_kernel<<<dim3(grid_for(n), W), 256, 0, s>>>(n, v, ldv, cm, w.d32, n);
     }
     GBLU_CK(ctx, cudaGetLastError(), "scale");
     // RBT factors: d := W1^T d / 2, LU solve, d := W2 d / 2 with (W1, W2) =
@@ -901,7 +901,7 @@ struct Solver {
     if (st) return st;
     {
       LaunchScope ls_(K_REFINE, 0.0, 0.0, s);
-      update_from_f32_kernel<<<dim3(grid_for(n), W), 256, 0, s>>>(n, W, out, ldo, w.d32, n, cm);
+      update_from_f32_kernel<<<dim3(grid_for(n), W), 256, 0, s>>>(n, out, ldo, w.d32, n, cm);
     }
     GBLU_CK(ctx, cudaGetLastError(), "update");
     return GBLU_OK;
