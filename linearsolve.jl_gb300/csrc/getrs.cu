@@ -281,7 +281,7 @@ solve_sweep_kernel(int64_t n, const T* __restrict__ LU, int64_t lda, const int32
             atomicCAS(&scr->error, 0, (int)DEV_TIMEOUT_SOLVE);
             give_up = true;
           }
-          if (give_up) break;  // the row warps see the error word
+          if (__any_sync(kAll, give_up)) break;  // the whole warp; the row warps see the error word
         }
       }
     }
