@@ -17,7 +17,10 @@
 // with correctly rounded reciprocals: without pivoting nothing bounds the
 // condition of U's diagonal blocks, and a product with the inverse of one leaves
 // an error of its condition times u in the rows below (8 w u |L||U| exceeded 400
-// times where the condition is 1.6^31).
+// times where the condition is 1.6^31).  With FP32 operands the factors have the
+// bits of 32-column leaves with their TRSMs and updates (n = 64 .. 3000).  A leaf
+// of n = 4096 takes the rows below 12.0 us in place of 9.8 (ncu, cold caches), and
+// the top block as much less without the inverses to form.
 //
 // An exactly zero pivot sets info and leaves its column unscaled, as getf2.
 #include <cuda_runtime.h>
